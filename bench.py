@@ -1167,7 +1167,7 @@ def adjoint_roofline(fst, ast, clocks, local):
         alu_peak = n_sm * 64 * sm_mhz * 1e6 / GATHER_INSTR_PER_PAIR / 1e9
         achieved = s.dipole_pairs / (s.gather_ms * 1e-3) / 1e9 if s.gather_ms else None
         kernel = "k_gather (forward dipole gathers)" if top.startswith("forward") else \
-            "k_gather_adjoint (the adjoint pass's dipole gathers: the MD5 chain replayed, derivatives of accepted pairs)"
+            "k_gather<true> (the adjoint pass's dipole gathers: the MD5 chain replayed, derivatives of accepted pairs)"
         out = {"bound": "alu", "kernel": kernel, "achieved": achieved, "peak": alu_peak, "unit": "Gpair/s",
                "frac": achieved / alu_peak if achieved else None,
                "peak_source": "INT32 pipe: 64 lanes/clk/SM x SMs x median SM clock / %d thread instructions per pair of the "

@@ -104,7 +104,8 @@ enum CounterSlot {
   CNT_FETCH_EXT = 9,     // slots 2..9 are reset at the start of each bounce,
   CNT_SHADOW = 10,       // 10..11 before its shading (the previous bounce's shadow rays may still run)
   CNT_FETCH_SH = 11,
-  CNT_GATHER = 12,
+  CNT_GATHER = 12,       // 12..13 are reset before the dipole gathers: paths that owe some, paths taken
+  CNT_FETCH_GATHER = 13,
   CNT_SEGMENTS_LO = 14,  // 64-bit totals as two words each at even slots (8-byte aligned atomicAdd on unsigned long long)
   CNT_SHADOW_TOTAL = 16,
   CNT_CAPPED = 18,

@@ -1683,7 +1683,7 @@ __device__ bool rough_translucent_vertex(const SceneDev& S, const WfDev& w, uint
 // own launch is writing.
 //
 // Adjoint: the gather a camera path owes at an entry vertex is taken off R there (its forward value
-// was stored with the path); its gradient is added at the end (k_gather_adj).  Inside, the weight
+// was stored with the path); its gradient is added at the end (k_gather<true>).  Inside, the weight
 // beam_T / p has p detached: d w / d sigma_a / w = -t * scale per channel.
 template <bool kAdj>
 __global__ void __launch_bounds__(kBlock) k_shade_translucent(WfDev w)
@@ -1813,238 +1813,307 @@ __global__ void __launch_bounds__(kBlock) k_gather_collect(WfDev w, uint64_t n_p
 // L != 0 of the path's frame and object: distance Russian roulette with p = exp(-dist * min sigma_tr)
 // on one MD5 draw, and on acceptance T12 * L * S(probe, xo) / p with the standard or directional
 // dipole.  The sum times global_coeff / samples is added to the path's radiance, weighted by the
-// throughput at the vertex.  One thread per path: the MD5 stream is one sequential chain.
+// throughput at the vertex.  The MD5 stream of a path is one sequential chain, so a lane owns a path.
 //
-// A differentiable forward render also stores each gather's value with the path (adj_G); the adjoint
-// replays the same gathers in k_gather_adjoint.
-__global__ void __launch_bounds__(kBlock) k_gather(WfDev w, SssDev g, const uint32_t* list)
-{
-  const uint32_t n = w.cnt[CNT_GATHER];
-  unsigned long long pairs = 0, gathers = 0;
-  for (uint32_t i = blockIdx.x * kBlock + threadIdx.x; i < n; i += gridDim.x * kBlock) {
-    uint32_t pid = list[i];
-    const ItemDev& it = w.items[w.path_item[pid]];
-    const SceneDev& S = w.scenes[it.scene];
-    uint4 rg = w.rng[pid];
-    uint2 t64 = make_uint2(rg.y, rg.z);
-    uint32_t fl = (uint32_t)((pid - it.path_begin) / it.pixels);
-    float4 r4 = w.rad[pid];
-    float3 L = ld3(r4);
-    const uint64_t gp = S.adj_G ? (uint64_t)(it.first_frame + fl - S.adj_first) * it.pixels + (pid - it.path_begin) % it.pixels : 0;
-    for (int slot = (int)(rg.w >> META_GSHIFT) - 1; slot >= 0; --slot) {
-      size_t at = (size_t)slot * w.cap + pid;
-      float4 a = w.g_a[at], b = w.g_b[at];
-      float2 c = w.g_c[at];
-      const int mat = __float_as_int(c.y);
-      if (mat < 0) {  // reset marker: the MD5 state the vertex below was entered with
-        t64 = make_uint2(__float_as_uint(a.x), __float_as_uint(a.y));
-        continue;
-      }
-      const float3 xo = ld3(a), no = ld3(b), thr = f3(a.w, b.w, c.x);
-      const float4 gd = w.g_d[at];
-      const bool rough = gd.w != 0.0f;  // rough boundary: draws must exceed 0.001, terms carry the weight
-      const float3 gw = ld3(gd);
-      const MatDev& m = S.mats[mat];
-      const ScatDev& P = S.scat[mat];
-      const uint32_t set_in_item = fl * S.n_trans + m.aux;
-      const size_t pb = it.probe_begin + (size_t)set_in_item * S.probe_samples;
-      const uint32_t nc = g.pc_cnt[it.set_begin + set_in_item];
-      const float chosen = fminf(P.transport.x, fminf(P.transport.y, P.transport.z));
-      float3 acc = f3s(0.0f);
-      if (m.model == DIRECTIONAL_DIPOLE) {
-        for (uint32_t k = 0; k < nc; ++k) {
-          float3 pos = ld3(__ldg(g.pc_pos + pb + k));
-          float dist = length(xo - pos);
-          float exp_term = expf(-dist * chosen);
-          const float rn = rnd_md5(t64);
-          if (rn < exp_term && (!rough || rn > 0.001f)) {
-            float3 wl = ld3(__ldg(g.pc_wl + pb + k));
-            float3 pn = ld3(__ldg(g.pc_nrm + pb + k)), pt = ld3(__ldg(g.pc_tr + pb + k));
-            float3 term = wl * dirpole_bssrdf(pos, pn, pt, xo, no, P) / exp_term;
-            acc = acc + (rough ? term * gw : term);
-          }
-        }
-      } else {
-        const StdDipole sd = std_dipole_terms(P);
-        for (uint32_t k = 0; k < nc; ++k) {
-          float3 pos = ld3(__ldg(g.pc_pos + pb + k));
-          float dist = length(xo - pos);
-          float exp_term = expf(-dist * chosen);
-          const float rn = rnd_md5(t64);
-          if (rn < exp_term && (!rough || rn > 0.001f)) {
-            float3 wl = ld3(__ldg(g.pc_wl + pb + k));
-            float3 term = wl * dipole_bssrdf(dist, sd) / exp_term;
-            acc = acc + (rough ? term * gw : term);
-          }
-        }
-      }
-      const float3 contrib = acc * P.global_coeff / (float)S.probe_samples;
-      L = L + thr * contrib;
-      if (S.adj_G) S.adj_G[gp * S.adj_slots + slot] = make_float4(contrib.x, contrib.y, contrib.z, 0.0f);
-      pairs += nc;
-      ++gathers;
-    }
-    w.rad[pid] = make_float4(L.x, L.y, L.z, r4.w);
-    w.rng[pid] = make_uint4(rg.x, t64.x, t64.y, rg.w);
-  }
-  if (pairs) atomicAdd(cnt64(w.cnt, CNT_PAIRS), pairs);
-  if (gathers) atomicAdd(cnt64(w.cnt, CNT_GATHERS), gathers);
-}
-
-// The adjoint gathers, warp by warp: lanes walk their paths' gathers and probes (one probe or one gather
-// set-up per step: distance, the detached acceptance test on one MD5 draw -- the same chain as the
-// forward gather), and every accepted pair of a differentiated material goes to the warp's queue in
-// shared memory; whenever 32 pairs are queued, the whole warp evaluates them, one pair per lane, the
-// standard dipole's derivatives with respect to sigma_a and sigma_s' per channel (dipole_channel_grad)
-// times the pair's weight * L / p and its gather's factor (image gradient x throughput x global_coeff /
-// samples), and adds them to the material's gradient buffer (one warp reduction and six atomics when
-// the 32 pairs share a material).  The derivative, the costly part, thus runs on full warps instead of
-// on the lanes that happened to accept a pair.
-struct AdjPair {
-  float dist, p;    // distance to the probe, acceptance probability exp_term
-  uint32_t wl;      // index of the probe's weight * L in pc_wl
-  uint32_t scene;   // the pair's scene in the pass
-  float3 f;         // factor of its gather
-  int mat;
+// What bounds it: the 64 MD5 steps are three ALU-pipe instructions each (logic, three-input add,
+// shift-and-add; 190 per draw counted by ncu), and the ALU pipe takes 64 lanes per clock and SM, so a
+// draw costs at least 3.0 clocks per SM.  The rest of a pair is kept off that pipe and out of the way:
+//  * the roulette is decided from the draw's upper 31 bits against an upper bound of p taken with the
+//    approximate square root and exponential (gather_bound); only the pairs that this bound cannot
+//    reject (the accepted ones and about one in 10^4 more) go through the exact test, which alone
+//    decides;
+//  * those pairs are queued per warp in shared memory and evaluated 32 at a time, one pair per lane,
+//    so that the dipole runs on full warps instead of on the lanes that happened to accept; a lane
+//    then adds the values of its own pairs in probe order, so the sum is the sequential one bit for bit;
+//  * a lane whose path is done takes the next path of the list at once, and the warp steps through the
+//    pairs without any test of the lanes' ends until the first of them is due;
+//  * the next probe is loaded before the draw and bounded after it;
+//  * the draw's additions run on the FMA pipe (md5_u2_split).
+// One thread per path with the exact test in the probe loop and the dipole on the accepting lanes took
+// 19.6 ms for 456,028 gathers of 3,011 pairs (512 x 512 x 4 frames, 4,096 probes: 69.9 Gpair/s); this
+// takes 16.2 ms (84.8).  Gathers of few pairs and many acceptances (175,143 of 312 pairs, scale 10): 3.04
+// to 1.27 ms.  Five blocks per SM: with 6 to 8 the evaluation spills and the times are the same or worse.
+//
+// A differentiable forward render also stores each gather's value with the path (adj_G).  kAdj: the
+// adjoint replays the same chain; a queued pair of a differentiated material adds the standard dipole's
+// derivatives with respect to sigma_a and sigma_s' per channel (dipole_channel_grad) times its weight *
+// L / p and its gather's factor (image gradient x throughput x global_coeff / samples) to the warp's sums
+// for the material's gradient buffer (GatherGrad).
+constexpr int kGatherQueue = 64;  // per warp; at most 31 + 32 entries are held
+struct GatherWarp {
+  uint4 q[kGatherQueue];   // queued pairs: owner lane, probe of its set, the draw's two words
+  float4 xo[32];           // per owner lane, its current gather: position, min sigma_tr
+  float4 f[32];            //   forward: boundary weight and rough flag; adjoint: factor
+  float4 no[32];           //   forward: normal
+  unsigned long long pb[32];  // first probe of the set
+  uint2 sm[32];            //   scene of the pass, material
+  float4 val[32];          // a flush's values and whether the pair was accepted
 };
-constexpr int kAdjQueue = 64;  // per warp; at most 31 + 32 entries are held
 
-__device__ __forceinline__ void adj_pairs_eval(const WfDev& w, const SssDev& g, const AdjPair* q, int count, int lane)
+// Upper bound, scaled by 2^31, of the acceptance probability exp(-dist(p, xo) * chosen) with c2 = chosen
+// * log2(e).  The approximate square root and exponential and the product's roundings are within 1e-5
+// relative while the probability is above 2^-32; the slack is 1e-4 relative plus 5 * 2^-31.  A NaN
+// anywhere gives NaN, which rejects nothing.
+__device__ __forceinline__ float gather_bound(const float4& p, const float3& xo, float c2)
 {
-  float3 ga = f3s(0.0f), gs = f3s(0.0f);
-  float* gr = nullptr;
-  if (lane < count) {
-    const AdjPair e = q[lane];
-    const SceneDev& S = w.scenes[e.scene];
-    const ScatDev& P = S.scat[e.mat];
-    const float scale = S.mats[e.mat].a.x;
-    gr = S.mat_grad[e.mat];
-    const float3 wl = ld3(__ldg(g.pc_wl + e.wl));
-    const Dual2 sx = dipole_channel_grad(e.dist, P.absorption.x, P.reducedExtinction.x, P.A.x, scale);
-    const Dual2 sy = dipole_channel_grad(e.dist, P.absorption.y, P.reducedExtinction.y, P.A.y, scale);
-    const Dual2 sz = dipole_channel_grad(e.dist, P.absorption.z, P.reducedExtinction.z, P.A.z, scale);
-    const float3 k = e.f * wl / e.p;
-    ga = k * f3(sx.da, sy.da, sz.da);
-    gs = k * f3(sx.ds, sy.ds, sz.ds);
-  }
-  const unsigned long long g0 = __shfl_sync(0xffffffffu, (unsigned long long)gr, 0);
-  if (__all_sync(0xffffffffu, lane >= count || (unsigned long long)gr == g0)) {
-    float v[6] = {ga.x, ga.y, ga.z, gs.x, gs.y, gs.z};
+  const float dx = xo.x - p.x, dy = xo.y - p.y, dz = xo.z - p.z;
+  const float d2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, dx * dx));
+  float dist, e;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(dist) : "f"(d2));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(dist * -c2));
+  return __fmaf_rn(e, 2147483648.0f * 1.0001f, 5.0f);
+}
+
+// Adjoint: what a warp has gathered for the gradient buffer `g` (6 floats), per lane.  A buffer takes
+// one warp reduction and six atomics when the warp turns to another material's buffer and at its end:
+// adding every flush's sum at once kept all warps waiting for the same six addresses.
+struct GatherGrad {
+  float* g = nullptr;
+  float v[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+};
+__device__ __forceinline__ void gather_grad_emit(GatherGrad& a, int lane)
+{
+  if (!a.g) return;
 #pragma unroll
-    for (int j = 0; j < 6; ++j)
-      for (int off = 16; off; off >>= 1) v[j] += __shfl_xor_sync(0xffffffffu, v[j], off);
-    if (lane == 0 && g0) {
-      float* d = (float*)g0;
-#pragma unroll
-      for (int j = 0; j < 6; ++j) atomicAdd(d + j, v[j]);
-    }
-  } else if (gr) {
-    atomicAdd(gr + 0, ga.x);
-    atomicAdd(gr + 1, ga.y);
-    atomicAdd(gr + 2, ga.z);
-    atomicAdd(gr + 3, gs.x);
-    atomicAdd(gr + 4, gs.y);
-    atomicAdd(gr + 5, gs.z);
+  for (int j = 0; j < 6; ++j) {
+    float r = a.v[j];
+    for (int off = 16; off; off >>= 1) r += __shfl_xor_sync(0xffffffffu, r, off);
+    if (lane == 0) atomicAdd(a.g + j, r);
+    a.v[j] = 0.0f;
   }
 }
 
-__global__ void __launch_bounds__(kBlock) k_gather_adjoint(WfDev w, SssDev g, const uint32_t* list)
+// Evaluates the first `count` queued pairs of the warp, one per lane.  Forward: adds the values of the
+// calling lane's own pairs (bits of `mine`, queue order = probe order) to acc.  Adjoint: adds the pair's
+// derivatives to grad.
+template <bool kAdj>
+__device__ __forceinline__ void gather_flush(const WfDev& w, const SssDev& g, GatherWarp& s, int count, int lane, unsigned mine, float3& acc,
+                                             GatherGrad& grad)
 {
-  __shared__ AdjPair queue[kWarps][kAdjQueue];
-  const uint32_t n = w.cnt[CNT_GATHER];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  AdjPair* q = queue[wid];
-  int qn = 0;  // warp-uniform
-  unsigned long long pairs = 0, gathers = 0;
-  for (uint32_t base = (blockIdx.x * kWarps + wid) * 32u; base < n; base += gridDim.x * kBlock) {
-    const uint32_t i = base + lane;
-    bool active = i < n;
-    uint32_t pid = 0, scene = 0, fl = 0, pb = 0, nc = 0, k = 0;
-    int slot = -1, mat = 0;
-    const ItemDev* it = nullptr;
-    const SceneDev* S = nullptr;
-    uint4 rg = make_uint4(0, 0, 0, 0);
-    uint2 t64 = make_uint2(0, 0);
-    float3 dl = f3s(0.0f), xo = f3s(0.0f), f = f3s(0.0f);
-    float chosen = 0.0f;
-    bool diff = false;
-    if (active) {
-      pid = list[i];
-      it = &w.items[w.path_item[pid]];
-      scene = it->scene;
-      S = &w.scenes[scene];
-      rg = w.rng[pid];
-      t64 = make_uint2(rg.y, rg.z);
-      fl = (uint32_t)((pid - it->path_begin) / it->pixels);
-      dl = ld3(w.adj_a[pid]);
-      slot = (int)(rg.w >> META_GSHIFT) - 1;
+  __syncwarp();
+  float3 v = f3s(0.0f), ds = f3s(0.0f);
+  float* gr = nullptr;
+  bool ok = false;
+  if (lane < count) {
+    const uint4 e = s.q[lane];
+    const uint32_t o = e.x;
+    const float4 x4 = s.xo[o], f4 = s.f[o];
+    const uint2 id = s.sm[o];
+    const SceneDev& S = w.scenes[id.x];
+    const ScatDev& P = S.scat[id.y];
+    const uint64_t at = s.pb[o] + e.y;
+    const float3 xo = ld3(x4);
+    const float3 pos = ld3(__ldg(g.pc_pos + at));
+    const float dist = length(xo - pos);
+    const float exp_term = expf(-dist * x4.w);
+    const float rn = md5_draw(e.z, e.w);
+    if constexpr (kAdj) {
+      ok = rn < exp_term;
+      if (ok) {
+        const float scale = S.mats[id.y].a.x;
+        gr = S.mat_grad[id.y];
+        const float3 wl = ld3(__ldg(g.pc_wl + at));
+        const Dual2 sx = dipole_channel_grad(dist, P.absorption.x, P.reducedExtinction.x, P.A.x, scale);
+        const Dual2 sy = dipole_channel_grad(dist, P.absorption.y, P.reducedExtinction.y, P.A.y, scale);
+        const Dual2 sz = dipole_channel_grad(dist, P.absorption.z, P.reducedExtinction.z, P.A.z, scale);
+        const float3 k = ld3(f4) * wl / exp_term;
+        v = k * f3(sx.da, sy.da, sz.da);
+        ds = k * f3(sx.ds, sy.ds, sz.ds);
+      }
+    } else {
+      const bool rough = f4.w != 0.0f;  // rough boundary: draws must exceed 0.001, terms carry the weight
+      ok = rn < exp_term && (!rough || rn > 0.001f);
+      if (ok) {
+        const float3 wl = ld3(__ldg(g.pc_wl + at));
+        float3 term;
+        if (S.mats[id.y].model == DIRECTIONAL_DIPOLE)
+          term = wl * dirpole_bssrdf(pos, ld3(__ldg(g.pc_nrm + at)), ld3(__ldg(g.pc_tr + at)), xo, ld3(s.no[o]), P) / exp_term;
+        else
+          term = wl * dipole_bssrdf(dist, std_dipole_terms(P)) / exp_term;
+        v = rough ? term * ld3(f4) : term;
+      }
     }
-    while (__any_sync(0xffffffffu, active)) {
-      bool want = false;
-      AdjPair e;
-      if (active) {
-        if (k >= nc) {  // the next gather of the path (or its end)
-          if (slot < 0) {
-            w.rng[pid] = make_uint4(rg.x, t64.x, t64.y, rg.w);
-            active = false;
-          } else {
-            const size_t at = (size_t)slot * w.cap + pid;
-            const float4 a = w.g_a[at], b = w.g_b[at];
-            const float2 c = w.g_c[at];
-            --slot;
-            mat = __float_as_int(c.y);
-            if (mat < 0) {  // reset marker: the MD5 state the vertex below was entered with
-              t64 = make_uint2(__float_as_uint(a.x), __float_as_uint(a.y));
-            } else {
-              xo = ld3(a);
-              const float3 thr = f3(a.w, b.w, c.x);
-              const MatDev& m = S->mats[mat];
-              const ScatDev& P = S->scat[mat];
-              const uint32_t set_in_item = fl * S->n_trans + m.aux;
-              pb = (uint32_t)(it->probe_begin + (size_t)set_in_item * S->probe_samples);
-              nc = g.pc_cnt[it->set_begin + set_in_item];
-              k = 0;
-              chosen = fminf(P.transport.x, fminf(P.transport.y, P.transport.z));
-              f = dl * thr * P.global_coeff / (float)S->probe_samples;
-              diff = S->mat_grad[mat] != nullptr;
-              pairs += nc;
-              ++gathers;
+  }
+  if constexpr (kAdj) {
+    const unsigned have = __ballot_sync(0xffffffffu, gr != nullptr);
+    if (have == 0) return;
+    const unsigned long long g0 = __shfl_sync(0xffffffffu, (unsigned long long)gr, __ffs(have) - 1);
+    if (__all_sync(0xffffffffu, gr == nullptr || (unsigned long long)gr == g0)) {
+      if ((unsigned long long)grad.g != g0) {
+        gather_grad_emit(grad, lane);
+        grad.g = (float*)g0;
+      }
+      grad.v[0] += v.x;
+      grad.v[1] += v.y;
+      grad.v[2] += v.z;
+      grad.v[3] += ds.x;
+      grad.v[4] += ds.y;
+      grad.v[5] += ds.z;
+    } else if (gr) {
+      atomicAdd(gr + 0, v.x);
+      atomicAdd(gr + 1, v.y);
+      atomicAdd(gr + 2, v.z);
+      atomicAdd(gr + 3, ds.x);
+      atomicAdd(gr + 4, ds.y);
+      atomicAdd(gr + 5, ds.z);
+    }
+  } else {
+    s.val[lane] = make_float4(v.x, v.y, v.z, ok ? 1.0f : 0.0f);
+    __syncwarp();
+    for (; mine; mine &= mine - 1) {
+      const float4 t = s.val[__ffs(mine) - 1];
+      if (t.w != 0.0f) acc = acc + ld3(t);
+    }
+  }
+}
+
+template <bool kAdj>
+__global__ void __launch_bounds__(kBlock, 5) k_gather(WfDev w, SssDev g, const uint32_t* list, uint32_t one)
+{
+  __shared__ GatherWarp shared[kWarps];
+  const uint32_t n = w.cnt[CNT_GATHER];
+  const int lane = threadIdx.x & 31;
+  GatherWarp& s = shared[threadIdx.x >> 5];
+  int qn = 0;                     // queued pairs (warp-uniform)
+  unsigned long long mine = 0;    // this lane's among them
+  unsigned long long pairs = 0, gathers = 0;
+  bool active = true, in_gather = false;
+  int slot = -1;                  // gathers of the path left below the current one
+  uint32_t pid = 0xffffffffu, k = 0, nc = 0;
+  uint2 t64 = make_uint2(0, 0);
+  float3 xo = f3s(0.0f), acc = f3s(0.0f);
+  float c2 = 0.0f, bound = 0.0f;
+  const float4* probes = g.pc_pos;
+  GatherGrad grad;
+  for (;;) {
+    // lanes at the end of a gather: its pending pairs, its sum, and the next gather of the path or the
+    // next path of the list
+    const bool end = active && k >= nc;
+    if (__any_sync(0xffffffffu, end && mine != 0)) {
+      for (; qn > 32; qn -= 32) {
+        gather_flush<kAdj>(w, g, s, 32, lane, (unsigned)mine, acc, grad);
+        mine >>= 32;
+        uint4 moved = make_uint4(0, 0, 0, 0);
+        if (lane < qn - 32) moved = s.q[32 + lane];
+        __syncwarp();
+        if (lane < qn - 32) s.q[lane] = moved;
+      }
+      gather_flush<kAdj>(w, g, s, qn, lane, (unsigned)mine, acc, grad);
+      mine = 0;
+      qn = 0;
+    }
+    if (end) {
+      for (;;) {
+        const ItemDev* it = nullptr;
+        const SceneDev* S = nullptr;
+        uint32_t fl = 0;
+        if (pid != 0xffffffffu) {
+          it = &w.items[w.path_item[pid]];
+          S = &w.scenes[it->scene];
+          fl = (uint32_t)((pid - it->path_begin) / it->pixels);
+        }
+        if (in_gather) {
+          in_gather = false;
+          if constexpr (!kAdj) {
+            const size_t at = (size_t)(slot + 1) * w.cap + pid;
+            const float3 thr = f3(w.g_a[at].w, w.g_b[at].w, w.g_c[at].x);
+            const float3 contrib = acc * S->scat[__float_as_int(w.g_c[at].y)].global_coeff / (float)S->probe_samples;
+            const float4 r = w.rad[pid];
+            const float3 L = ld3(r) + thr * contrib;
+            w.rad[pid] = make_float4(L.x, L.y, L.z, r.w);
+            if (S->adj_G) {
+              const uint64_t gp = (uint64_t)(it->first_frame + fl - S->adj_first) * it->pixels + (pid - it->path_begin) % it->pixels;
+              S->adj_G[gp * S->adj_slots + slot + 1] = make_float4(contrib.x, contrib.y, contrib.z, 0.0f);
             }
           }
-        } else {  // one probe of the gather
-          const float3 pos = ld3(__ldg(g.pc_pos + pb + k));
-          const float dist = length(xo - pos);
-          const float exp_term = expf(-dist * chosen);
-          if (rnd_md5(t64) < exp_term && diff) {
-            want = true;
-            e.dist = dist;
-            e.p = exp_term;
-            e.wl = pb + k;
-            e.scene = scene;
-            e.f = f;
-            e.mat = mat;
-          }
-          ++k;
         }
-      }
-      const unsigned m = __ballot_sync(0xffffffffu, want);
-      if (want) q[qn + __popc(m & lanemask_lt())] = e;
-      qn += __popc(m);
-      __syncwarp();
-      if (qn >= 32) {
-        adj_pairs_eval(w, g, q, 32, lane);
-        __syncwarp();
-        const int rest = qn - 32;
-        AdjPair moved;
-        if (lane < rest) moved = q[32 + lane];
-        __syncwarp();
-        if (lane < rest) q[lane] = moved;
-        qn = rest;
-        __syncwarp();
+        if (slot < 0) {
+          if (pid != 0xffffffffu) {
+            const uint4 rg = w.rng[pid];
+            w.rng[pid] = make_uint4(rg.x, t64.x, t64.y, rg.w);
+          }
+          const uint32_t i = atomicAdd(w.cnt + CNT_FETCH_GATHER, 1u);
+          if (i >= n) {
+            active = false;
+            pid = 0xffffffffu;
+            break;
+          }
+          pid = list[i];
+          const uint4 rg = w.rng[pid];
+          t64 = make_uint2(rg.y, rg.z);
+          slot = (int)(rg.w >> META_GSHIFT) - 1;
+          continue;
+        }
+        const size_t at = (size_t)slot * w.cap + pid;
+        --slot;
+        const float4 a = w.g_a[at];
+        const int mat = __float_as_int(w.g_c[at].y);
+        if (mat < 0) {  // reset marker: the MD5 state the vertex below was entered with
+          t64 = make_uint2(__float_as_uint(a.x), __float_as_uint(a.y));
+          continue;
+        }
+        const ScatDev& P = S->scat[mat];
+        const uint32_t set_in_item = fl * S->n_trans + S->mats[mat].aux;
+        const uint64_t pb = it->probe_begin + (uint64_t)set_in_item * S->probe_samples;
+        const float chosen = fminf(P.transport.x, fminf(P.transport.y, P.transport.z));
+        nc = g.pc_cnt[it->set_begin + set_in_item];
+        k = 0;
+        acc = f3s(0.0f);
+        in_gather = true;
+        pairs += nc;
+        ++gathers;
+        if (nc == 0) continue;
+        xo = ld3(a);
+        c2 = chosen * 1.44269504f;
+        probes = g.pc_pos + pb;
+        s.xo[lane] = make_float4(xo.x, xo.y, xo.z, chosen);
+        s.pb[lane] = pb;
+        s.sm[lane] = make_uint2(it->scene, (uint32_t)mat);
+        bound = gather_bound(__ldg(probes), xo, c2);
+        if constexpr (kAdj) {
+          const float3 thr = f3(a.w, w.g_b[at].w, w.g_c[at].x);
+          const float3 f = ld3(w.adj_a[pid]) * thr * P.global_coeff / (float)S->probe_samples;
+          s.f[lane] = make_float4(f.x, f.y, f.z, S->mat_grad[mat] ? 1.0f : 0.0f);
+        } else {
+          s.f[lane] = w.g_d[at];
+          s.no[lane] = w.g_b[at];
+        }
+        break;
       }
     }
+    if (!__any_sync(0xffffffffu, active)) break;
+    // the adjoint queues the pairs of differentiated materials only
+    const bool take = active && (!kAdj || s.f[lane].w != 0.0f);
+    const uint32_t step = active ? 1u : 0u;
+    for (uint32_t rem = __reduce_min_sync(0xffffffffu, active ? nc - k : 0xffffffffu); rem; --rem) {
+      const float4 next = __ldg(probes + (k + step));
+      uint32_t h0, h1;
+      md5_u2_split(t64.x, t64.y, one, h0, h1);
+      t64 = make_uint2(h0, h1);
+      const bool cand = take && !((float)(int)(h1 & 0x7fffffffu) > bound);
+      const unsigned m = __ballot_sync(0xffffffffu, cand);
+      if (m) {
+        if (cand) {
+          const int at = qn + __popc(m & lanemask_lt());
+          s.q[at] = make_uint4((uint32_t)lane, k, h0, h1);
+          mine |= 1ull << at;
+        }
+        qn += __popc(m);
+        if (qn >= 32) {
+          gather_flush<kAdj>(w, g, s, 32, lane, (unsigned)mine, acc, grad);
+          mine >>= 32;
+          qn -= 32;
+          uint4 moved = make_uint4(0, 0, 0, 0);
+          if (lane < qn) moved = s.q[32 + lane];
+          __syncwarp();
+          if (lane < qn) s.q[lane] = moved;
+        }
+      }
+      bound = gather_bound(next, xo, c2);
+      k += step;
+    }
   }
-  if (qn > 0) adj_pairs_eval(w, g, q, qn, lane);
+  if constexpr (kAdj) gather_grad_emit(grad, lane);
   if (pairs) atomicAdd(cnt64(w.cnt, CNT_PAIRS), pairs);
   if (gathers) atomicAdd(cnt64(w.cnt, CNT_GATHERS), gathers);
 }
@@ -2344,7 +2413,8 @@ static pt_status ensure_sss(Context& c, uint64_t cap, uint32_t slots, uint64_t r
   }
   if (wf.probe_cap < records || !wf.probes.p) {
     st = wf.probes.reserve(records * 80, "probe records");
-    if (st == PT_OK) st = wf.pc_pos.reserve(records * sizeof(float4), "compacted probes");
+    // one position more than there are probes: the gathers load the probe after the one they draw for
+    if (st == PT_OK) st = wf.pc_pos.reserve((records + 1) * sizeof(float4), "compacted probes");
     if (st == PT_OK) st = wf.pc_wl.reserve(records * sizeof(float4), "compacted probes");
     if (st == PT_OK) st = wf.pc_nrm.reserve(records * sizeof(float4), "compacted probes");
     if (st == PT_OK) st = wf.pc_tr.reserve(records * sizeof(float4), "compacted probes");
@@ -2617,7 +2687,7 @@ pt_status launch_pass(Context& E, const PassLayout& L, const std::vector<SceneDe
     g.pc_tr = wf0.pc_tr.as<float4>();
     g.pc_cnt = wf0.pc_cnt.as<uint32_t>();
   }
-  const int grid_trace = sm_count() * 8, grid_shade = sm_count() * 8;
+  const int grid_trace = sm_count() * 8;
   // the 4-wide BVH when every scene of the pass has one (pass_resources)
   const bool w4 = E.pass_w4;
   // persistent grids: the SM count times the resident blocks of the single- and multi-scene kernels
@@ -2828,12 +2898,12 @@ pt_status launch_pass(Context& E, const PassLayout& L, const std::vector<SceneDe
     count_launch();
     if ((st = bounces(adjoint)) != PT_OK) return st;
     if (n_probes) {
-      PT_CHECK_CUDA(cudaMemsetAsync(w.cnt + CNT_GATHER, 0, 4, s_main), "reset gather list");
+      PT_CHECK_CUDA(cudaMemsetAsync(w.cnt + CNT_GATHER, 0, 8, s_main), "reset gather list");
       uint32_t* list = wf->q_a.as<uint32_t>();
       k_gather_collect<<<grid_for(n_paths, kBlock, 16), kBlock, 0, s_main>>>(w, n_paths, list);
       if ((st = prof_begin(PROF_GATHER)) != PT_OK) return st;
-      if (adjoint) k_gather_adjoint<<<grid_shade, kBlock, 0, s_main>>>(w, g, list);
-      else k_gather<<<grid_shade, kBlock, 0, s_main>>>(w, g, list);
+      if (adjoint) k_gather<true><<<full_wave(k_gather<true>), kBlock, 0, s_main>>>(w, g, list, 1u);
+      else k_gather<false><<<full_wave(k_gather<false>), kBlock, 0, s_main>>>(w, g, list, 1u);
       if ((st = prof_end()) != PT_OK) return st;
       count_launch(2);
     }
