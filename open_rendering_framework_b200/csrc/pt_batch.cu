@@ -55,6 +55,7 @@ std::vector<uint64_t> graph_key(const Context& E, const PassLayout& L, const std
   k.push_back(L.sss ? 1 : 0);
   k.push_back(L.layered ? 1 : 0);
   k.push_back(L.ms ? 1 : 0);
+  k.push_back(L.rough ? 1 : 0);
   k.push_back(L.g_slots);
   k.push_back(L.items.size());
   for (size_t i = 0; i < L.chunk_paths.size(); ++i) {
@@ -73,6 +74,7 @@ std::vector<uint64_t> graph_key(const Context& E, const PassLayout& L, const std
   k.push_back((uint64_t)E.opt.bin_items);
   k.push_back((uint64_t)E.opt.overlap);
   k.push_back((uint64_t)E.opt.dual);
+  k.push_back((uint64_t)E.opt.pool);
   k.push_back((uint64_t)L.dual);
   k.push_back((uint64_t)E.pass_w4);
   return k;

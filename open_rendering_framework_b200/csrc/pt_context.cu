@@ -940,6 +940,9 @@ pt_status pt_set_option(pt_ctx* ctx, const char* name, int64_t value)
   } else if (k == "dual") {
     if (value != 0 && value != 1) return fail(PT_INVALID_ARG, "pt_set_option: dual must be 0 or 1");
     ctx->c.opt.dual = (int)value;
+  } else if (k == "pool") {
+    if (value < 0 || value > 2) return fail(PT_INVALID_ARG, "pt_set_option: pool must be 0, 1 or 2");
+    ctx->c.opt.pool = (int)value;
   } else if (k == "overlap") {
     if (value != 0 && value != 1) return fail(PT_INVALID_ARG, "pt_set_option: overlap must be 0 or 1");
     ctx->c.opt.overlap = (int)value;

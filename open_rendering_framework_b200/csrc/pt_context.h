@@ -143,6 +143,7 @@ struct SceneFacts {
   int max_depth = 0;
   bool layered = false;  // has a material of queue class QC_LAYERED
   bool ms = false;       // has a conductor or rough dielectric of the multiple-scattering model
+  bool rough = false;    // has a rough translucent material
 };
 // A request: frames [first_frame, first_frame + n_frames) of scene `scene`.
 struct ItemReq {
@@ -160,6 +161,7 @@ struct PassLayout {
   bool dual = false;     // chunks alternate between two wavefronts that run at once (two pipelines)
   bool layered = false;  // some scene of the pass has layered materials (k_shade_layered is launched)
   bool ms = false;       // some scene of the pass has multiple-scattering conductors or dielectrics
+  bool rough = false;    // some scene of the pass has rough translucent materials
   uint32_t g_slots = 0;
 };
 
@@ -174,6 +176,7 @@ struct Options {
                         // bounce's extend and binning; 0: every launch in order on the context stream
   int dual = 1;         // 1: passes without translucent materials split their paths into chunks of half the
                         // wavefront that run two at a time on two wavefronts (two pipelines); 0: one wavefront
+  int pool = 1;         // 1: passes of few paths run all bounces in one launch of path pools; 0: never; 2: always
 };
 
 struct Context {

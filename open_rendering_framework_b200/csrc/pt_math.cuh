@@ -72,10 +72,19 @@ PT_HD uint32_t tea16(uint32_t v0, uint32_t v1)
   }
   return v0;
 }
-// tea_hash / rnd_tea, random.h:117-127 (the draw may round up to exactly 1.0f).
+// tea_hash / rnd_tea, random.h:117-127 (the draw may round up to exactly 1.0f).  A draw is about 160
+// instructions inlined; a translation unit whose kernels hold many beside other large code defines
+// PT_TEA_CALL to have one copy called instead (a diffuse vertex alone inlines seven, 18 KB).
+#ifdef PT_TEA_CALL
+static __device__ __noinline__ uint32_t tea_call(uint32_t v) { return tea16(v, 100u); }
+#endif
 PT_HD float rnd_tea(uint32_t& prev)
 {
+#if defined(PT_TEA_CALL) && defined(__CUDA_ARCH__)
+  prev = tea_call(prev);
+#else
   prev = tea16(prev, 100u);
+#endif
   return (float)(prev & 0x7FFFFFFFu) / (float)0x80000000u;
 }
 // lcg / rnd, random.h:43-61.
