@@ -296,6 +296,113 @@ __global__ void k_trace_any(SceneDev S, const float4* ot, const float4* dt, uint
   }
 }
 
+// The same queries over the 4-wide BVH: a warp owns a run of `per` rays and keeps 32 of them in flight,
+// giving a finished lane the run's next ray once `kQueryRefill` lanes are idle (the persistent traversal of
+// the renders, without its queue).  A ray that wide_ray refuses is traced over the BVH2 when it is taken.
+// Bound by the latency of dependent node loads and by lanes of unequal length, as the renders' traversal.
+// 1,000,003 incoherent rays in a scene of 25,614 triangles, closest and any hit: 185 us against 568 us one
+// ray per thread over the BVH2.
+constexpr int kQueryRefill = 20;  // as the renders' traversal (their sweep: 16 to 22 within 1 %)
+constexpr int kQueryBlock = 128;
+template <bool kAny>
+__global__ void __launch_bounds__(kQueryBlock, 1024 / kQueryBlock) k_trace_wide(SceneDev S, const float4* ot, const float4* dt, uint32_t n,
+                                                                                uint32_t per, int32_t* out, float* tout, float* bary)
+{
+  __shared__ uint2 stk[kRing4 * kQueryBlock];
+  const TravGeom g = trav_geom(S);
+  const unsigned lane = threadIdx.x & 31, below = (1u << lane) - 1u;
+  const uint64_t warp = (uint64_t)blockIdx.x * (kQueryBlock / 32) + (threadIdx.x >> 5);
+  uint32_t next = (uint32_t)min(warp * per, (uint64_t)n);
+  const uint32_t end = (uint32_t)min(warp * per + per, (uint64_t)n);
+  bool has = false;
+  uint32_t i = 0;
+  float3 o = f3s(0.0f), d = f3s(0.0f);
+  float tmin = 0.0f, tmax = 0.0f;
+  RayPre4 rp{};
+  Hit h;
+  h.t = h.u = h.v = 0.0f;
+  h.prim = -1;
+  uint2 spill4[kSpill4];
+  Stack4 s4;
+  stack4_init(s4, stk + threadIdx.x, kQueryBlock, spill4);
+  int cur = kDone4;
+  for (;;) {
+    const unsigned idle = __ballot_sync(0xffffffffu, !has);
+    if (next < end && (__popc(idle) >= kQueryRefill || idle == 0xffffffffu)) {
+      const uint64_t at = (uint64_t)next + __popc(idle & below);
+      if (!has && at < end) {
+        i = (uint32_t)at;
+        const float4 a = __ldg(ot + i), b = __ldg(dt + i);
+        o = ld3(a);
+        d = ld3(b);
+        tmin = a.w;
+        tmax = b.w;
+        h.t = tmax;
+        h.u = h.v = 0.0f;
+        h.prim = -1;
+        if (wide_ray(o, d, tmin, g.trav_scale)) {
+          rp = ray_pre4(o, d, g.trav_scale);
+          stack4_init(s4, stk + threadIdx.x, kQueryBlock, spill4);
+          cur = 0;
+        } else {
+          if constexpr (kAny) h.prim = trace_any(g, o, d, tmin, tmax) ? 0 : -1;
+          else h = trace_closest(g, o, d, tmin, tmax);
+          cur = kDone4;
+        }
+        has = true;
+      }
+      next = (uint32_t)min((uint64_t)next + __popc(idle), (uint64_t)end);
+    }
+    if (__ballot_sync(0xffffffffu, has) == 0) break;
+    for (;;) {
+      const bool lp = has && cur < 0;
+      const bool np = has && cur >= 0 && cur != kDone4;
+      const unsigned lmask = __ballot_sync(0xffffffffu, lp), nmask = __ballot_sync(0xffffffffu, np);
+      if (lmask && (nmask == 0 || (kAny ? 2 * __popc(lmask) >= __popc(nmask) : __popc(lmask) >= 2 * __popc(nmask)))) {
+        if (lp) {
+          if constexpr (kAny) {
+            if (leaf_any(g, (uint32_t)cur, o, d, tmin, tmax)) {
+              h.prim = 0;
+              cur = kDone4;
+            } else {
+              cur = stack4_next(s4, tmax, false);
+            }
+          } else {
+            leaf_closest(g, (uint32_t)cur, o, d, tmin, h);
+            cur = stack4_next(s4, h.t, true);
+          }
+        }
+      } else if (np) {
+        if constexpr (kAny) cur = trav4_node_any(g, cur, rp, tmin, tmax, s4);
+        else cur = trav4_node_closest(g, cur, rp, tmin, h, s4);
+      }
+      const unsigned fin = __ballot_sync(0xffffffffu, !has || cur == kDone4);
+      if (fin == 0xffffffffu || (next < end && __popc(fin) >= kQueryRefill)) break;
+    }
+    if (has && cur == kDone4) {
+      if constexpr (kAny) {
+        out[i] = h.prim >= 0 || (S.n_ana && ana_any(S, o, d, tmin, tmax)) ? 1 : 0;
+      } else {
+        if (S.n_ana) ana_closest(S, o, d, tmin, h);
+        out[i] = h.prim;
+        tout[i] = h.prim >= 0 ? h.t : -1.0f;
+        bary[2 * i] = h.u;
+        bary[2 * i + 1] = h.v;
+      }
+      has = false;
+    }
+  }
+}
+template <bool kAny>
+static void launch_trace_wide(const Context& c, const SceneDev& S, const float* o, const float* d, uint32_t n, int32_t* out, float* t, float* bary)
+{
+  // one resident wave of warps, each with an equal run of rays, at least 32
+  const uint32_t warps = (uint32_t)sm_count() * 32u;
+  const uint32_t per = std::max(32u, (n + warps - 1) / warps);
+  const uint32_t blocks = (uint32_t)(((uint64_t)n + (uint64_t)per * (kQueryBlock / 32) - 1) / ((uint64_t)per * (kQueryBlock / 32)));
+  k_trace_wide<kAny><<<blocks, kQueryBlock, 0, c.stream>>>(S, (const float4*)o, (const float4*)d, n, per, out, t, bary);
+}
+
 // ------------------------------------------------------------------ environment CDFs (env_cameras.cu:23-75)
 // env_luminance_camera: luminance_NTSC(texel at the texel centre) * sin(theta).
 __global__ void k_env_luminance(EnvDev E, float* lum)
@@ -1017,7 +1124,9 @@ pt_status pt_trace_closest(pt_ctx* ctx, const float* d_orig_tmin, const float* d
   if (!c.built) return fail(PT_NOT_READY, "pt_trace_closest: call pt_build first");
   if (n == 0) return PT_OK;
   if (!d_orig_tmin || !d_dir_tmax || !d_prim || !d_t || !d_bary) return fail(PT_INVALID_ARG, "pt_trace_closest: null pointer");
-  k_trace_closest<<<grid_for(n, 128, 16), 128, 0, c.stream>>>(c.view(), (const float4*)d_orig_tmin, (const float4*)d_dir_tmax, n, d_prim, d_t, d_bary);
+  const SceneDev S = c.view();
+  if (S.nodes4) launch_trace_wide<false>(c, S, d_orig_tmin, d_dir_tmax, n, d_prim, d_t, d_bary);
+  else k_trace_closest<<<grid_for(n, 128, 16), 128, 0, c.stream>>>(S, (const float4*)d_orig_tmin, (const float4*)d_dir_tmax, n, d_prim, d_t, d_bary);
   count_launch();
   PT_CHECK_CUDA(cudaGetLastError(), "pt_trace_closest launch");
   return PT_OK;
@@ -1030,7 +1139,9 @@ pt_status pt_trace_any(pt_ctx* ctx, const float* d_orig_tmin, const float* d_dir
   if (!c.built) return fail(PT_NOT_READY, "pt_trace_any: call pt_build first");
   if (n == 0) return PT_OK;
   if (!d_orig_tmin || !d_dir_tmax || !d_hit) return fail(PT_INVALID_ARG, "pt_trace_any: null pointer");
-  k_trace_any<<<grid_for(n, 128, 16), 128, 0, c.stream>>>(c.view(), (const float4*)d_orig_tmin, (const float4*)d_dir_tmax, n, d_hit);
+  const SceneDev S = c.view();
+  if (S.nodes4) launch_trace_wide<true>(c, S, d_orig_tmin, d_dir_tmax, n, d_hit, nullptr, nullptr);
+  else k_trace_any<<<grid_for(n, 128, 16), 128, 0, c.stream>>>(S, (const float4*)d_orig_tmin, (const float4*)d_dir_tmax, n, d_hit);
   count_launch();
   PT_CHECK_CUDA(cudaGetLastError(), "pt_trace_any launch");
   return PT_OK;

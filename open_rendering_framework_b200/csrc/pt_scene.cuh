@@ -805,6 +805,18 @@ template <class G> PT_HD int trav4_node_any(const G& S, int cur, const RayPre4& 
   return next != kDone4 ? next : stack4_next(stk, tmax, false);
 }
 
+// Whether the wide BVH's box tests keep every box a ray can hit a triangle in.  ray_pre4 takes a
+// direction component below 2^-64 as +-2^-64, which the boxes' absolute margin covers up to t = 2^24, so
+// the scene must end before that; a relative slack on a negative distance would shrink the interval; and
+// every constant must be finite.  A NaN anywhere says no.  Other rays take the BVH2, whose reciprocals
+// are exact.
+PT_HD bool wide_ray(const float3& o, const float3& d, float tmin, float scale)
+{
+  const float om = fmaxf(fmaxf(fabsf(o.x), fabsf(o.y)), fabsf(o.z)), dm = fmaxf(fmaxf(fabsf(d.x), fabsf(d.y)), fabsf(d.z));
+  const bool finite = o.x - o.x == 0.0f && o.y - o.y == 0.0f && o.z - o.z == 0.0f && d.x - d.x == 0.0f && d.y - d.y == 0.0f && d.z - d.z == 0.0f;
+  return finite && tmin >= 0.0f && om <= kInvMax && dm <= kInvMax && dm * 16777216.0f >= om + 2.0f * scale;
+}
+
 template <class G> PT_HD Hit trace_closest(const G& S, const float3& o, const float3& d, float tmin, float tmax)
 {
   Hit h;
