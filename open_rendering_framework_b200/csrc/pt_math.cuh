@@ -72,15 +72,18 @@ PT_HD uint32_t tea16(uint32_t v0, uint32_t v1)
   }
   return v0;
 }
-// tea_hash / rnd_tea, random.h:117-127 (the draw may round up to exactly 1.0f).  A draw is about 160
-// instructions inlined; a translation unit whose kernels hold many beside other large code defines
-// PT_TEA_CALL to have one copy called instead (a diffuse vertex alone inlines seven, 18 KB).
-#ifdef PT_TEA_CALL
+// PT_OUTLINE_TEA, PT_OUTLINE_WALK: translation units whose kernels hold many draws, or several walks, beside
+// other large code define these to have one copy called -- of the draw (about 160 instructions inlined; a
+// diffuse vertex alone holds seven, 18 KB), and of the visible-normal sampler and its density and the walk's
+// height sampler and masking -- where inlined copies overflow the instruction cache.
+//
+// tea_hash / rnd_tea, random.h:117-127 (the draw may round up to exactly 1.0f).
+#ifdef PT_OUTLINE_TEA
 static __device__ __noinline__ uint32_t tea_call(uint32_t v) { return tea16(v, 100u); }
 #endif
 PT_HD float rnd_tea(uint32_t& prev)
 {
-#if defined(PT_TEA_CALL) && defined(__CUDA_ARCH__)
+#if defined(PT_OUTLINE_TEA) && defined(__CUDA_ARCH__)
   prev = tea_call(prev);
 #else
   prev = tea16(prev, 100u);
@@ -642,7 +645,7 @@ PT_D float bk_distribution(const float3& m, const float3& n, float alpha)  // :7
 
 // ------------------------------------------------------------------ distribution dispatch
 // GGX :190-207 / Beckmann :213-231 (identical apart from the slope sampler).
-PT_D float3 sample_vndf(uint32_t dist, const float3& wi, float ax, float ay, float z1, float z2, int* capped)
+PT_D float3 sample_vndf_inline(uint32_t dist, const float3& wi, float ax, float ay, float z1, float z2, int* capped)
 {
   float3 w11 = normalize(f3(ax * wi.x, ay * wi.y, wi.z));
   float th = acosf(w11.z);
@@ -659,10 +662,37 @@ PT_D float3 sample_vndf(uint32_t dist, const float3& wi, float ax, float ay, flo
   }
   return normalize(f3(-sx, -sy, 1.0f));
 }
-PT_D float eval_vndf(uint32_t dist, const float3& wi, const float3& wm, float ax, float ay)
+PT_D float eval_vndf_inline(uint32_t dist, const float3& wi, const float3& wm, float ax, float ay)
 {
   return dist == GGX ? ggx_eval_vndf(wi, wm, ax, ay) : bk_eval_vndf(wi, wm, ax, ay);
 }
+#if defined(PT_OUTLINE_WALK)
+struct VndfSample { float3 m; int capped; };
+static __device__ __noinline__ VndfSample sample_vndf_call(uint32_t dist, float3 wi, float ax, float ay, float z1, float z2)
+{
+  VndfSample r;
+  r.capped = 0;
+  r.m = sample_vndf_inline(dist, wi, ax, ay, z1, z2, &r.capped);
+  return r;
+}
+static __device__ __noinline__ float eval_vndf_call(uint32_t dist, float3 wi, float3 wm, float ax, float ay)
+{
+  return eval_vndf_inline(dist, wi, wm, ax, ay);
+}
+PT_D float3 sample_vndf(uint32_t dist, const float3& wi, float ax, float ay, float z1, float z2, int* capped)
+{
+  const VndfSample r = sample_vndf_call(dist, wi, ax, ay, z1, z2);
+  if (r.capped) *capped = 1;
+  return r.m;
+}
+PT_D float eval_vndf(uint32_t dist, const float3& wi, const float3& wm, float ax, float ay) { return eval_vndf_call(dist, wi, wm, ax, ay); }
+#else
+PT_D float3 sample_vndf(uint32_t dist, const float3& wi, float ax, float ay, float z1, float z2, int* capped)
+{
+  return sample_vndf_inline(dist, wi, ax, ay, z1, z2, capped);
+}
+PT_D float eval_vndf(uint32_t dist, const float3& wi, const float3& wm, float ax, float ay) { return eval_vndf_inline(dist, wi, wm, ax, ay); }
+#endif
 // Microfacet.h:76-87 and :89-101.
 PT_D float3 sample_visible_normal(uint32_t dist, const float3& wi, const float3& n, float ax, float ay, float z1, float z2, int* capped)
 {
@@ -703,7 +733,7 @@ PT_D float walter_bsdf(uint32_t dist, const float3& wi, const float3& wo, const 
 }
 
 // ------------------------------------------------------------------ multiscattering walks
-PT_D float sample_height(uint32_t dist, const float3& wr, float hr, float z, float ax, float ay)
+PT_D float sample_height_inline(uint32_t dist, const float3& wr, float hr, float z, float ax, float ay)
 {
   if (dist == GGX) {  // MicrofacetGGX.h:254-276
     if (wr.z > 0.9999f) return kDefaultMax;
@@ -723,17 +753,31 @@ PT_D float sample_height(uint32_t dist, const float3& wr, float hr, float z, flo
   float p = powf(1.0f - z, 1.0f / bk_lambda(wr, ax, ay));
   return gauss_inv_cdf(gcdf / p);
 }
-PT_D float G_height(uint32_t dist, const float3& wi, float h, float ax, float ay)
+PT_D float G_height_inline(uint32_t dist, const float3& wi, float h, float ax, float ay)
 {
   return dist == GGX ? ggx_G_height(wi, h, ax, ay) : bk_G_height(wi, h, ax, ay);
 }
+#if defined(PT_OUTLINE_WALK)
+static __device__ __noinline__ float sample_height(uint32_t dist, float3 wr, float hr, float z, float ax, float ay)
+{
+  return sample_height_inline(dist, wr, hr, z, ax, ay);
+}
+static __device__ __noinline__ float G_height(uint32_t dist, float3 wi, float h, float ax, float ay) { return G_height_inline(dist, wi, h, ax, ay); }
+#else
+PT_D float sample_height(uint32_t dist, const float3& wr, float hr, float z, float ax, float ay)
+{
+  return sample_height_inline(dist, wr, hr, z, ax, ay);
+}
+PT_D float G_height(uint32_t dist, const float3& wi, float h, float ax, float ay) { return G_height_inline(dist, wi, h, ax, ay); }
+#endif
 // Dielectric phase sample, GGX :279-304 / Beckmann :310-338.
 PT_D float3 sample_dielectric_phase(uint32_t dist, const float3& wi, float3& wm, float m_eta, uint32_t& seed, bool wi_out,
                                     bool& wo_out, float ax, float ay, int* capped)
 {
   float z1 = rnd_tea(seed), z2 = rnd_tea(seed);
   float eta = wi_out ? m_eta : 1.0f / m_eta;
-  wm = wi_out ? sample_vndf(dist, wi, ax, ay, z1, z2, capped) : -sample_vndf(dist, -wi, ax, ay, z1, z2, capped);
+  wm = sample_vndf(dist, wi_out ? wi : -wi, ax, ay, z1, z2, capped);
+  if (!wi_out) wm = -wm;
   float ct = fabsf(dot(wm, wi));
   float st2 = eta * eta * (1.0f - ct * ct);
   float ctt = sqrtf(1.0f - st2);
@@ -746,19 +790,24 @@ PT_D float3 sample_dielectric_phase(uint32_t dist, const float3& wi, float3& wm,
 PT_D float eval_dielectric_phase(uint32_t dist, const float3& wi, const float3& wo, bool wi_out, bool wo_out, float m_eta, float ax, float ay)
 {
   float eta = wi_out ? m_eta : 1.0f / m_eta;
-  if (wi_out == wo_out) {
-    float3 wh = normalize(wi + wo);
-    float D = wi_out ? eval_vndf(dist, wi, wh, ax, ay) : eval_vndf(dist, -wi, -wh, ax, ay);
-    float F = wi_out ? fresnel_R(wi, wh, eta) : fresnel_R(-wi, -wh, eta);
-    float a = wi_out ? 0.25f / dot(wi, wh) : 0.25f / dot(-wi, -wh);
+  const bool refl = wi_out == wo_out;
+  float3 wh;
+  if (refl) {
+    wh = normalize(wi + wo);
+  } else {
+    wh = -normalize(wi + wo / eta);
+    float sg = wi_out ? wh.z / fabsf(wh.z) : -wh.z / fabsf(wh.z);
+    wh = wh * sg;
+    if (dot(wh, wi) < 0.0f) return 0.0f;
+  }
+  // from inside, the reference mirrors both directions: the density of -wh seen from -wi (the Fresnel term
+  // and the dot products of two mirrored directions are the same numbers)
+  float D = eval_vndf(dist, wi_out ? wi : -wi, wi_out ? wh : -wh, ax, ay);
+  float F = fresnel_R(wi, wh, eta);
+  if (refl) {
+    float a = 0.25f / dot(wi, wh);
     return F * D * a;
   }
-  float3 wh = -normalize(wi + wo / eta);
-  float sg = wi_out ? wh.z / fabsf(wh.z) : -wh.z / fabsf(wh.z);
-  wh = wh * sg;
-  if (dot(wh, wi) < 0.0f) return 0.0f;
-  float D = wi_out ? eval_vndf(dist, wi, wh, ax, ay) : eval_vndf(dist, -wi, -wh, ax, ay);
-  float F = wi_out ? fresnel_R(wi, wh, eta) : fresnel_R(-wi, -wh, eta);
   float b = 1.0f / (eta * eta);
   float c = wi_out ? fmaxf(0.0f, -dot(wo, wh)) : fmaxf(0.0f, -dot(-wo, -wh));
   float e = wi_out ? dot(wi, wh) + dot(wo, wh) / eta : dot(-wi, -wh) + dot(-wo, -wh) / eta;
@@ -812,7 +861,8 @@ PT_D float3 ms_dielectric_sample(uint32_t dist, const float3& lwi, float eta, fl
   for (int it = 0;; ++it) {
     if (it >= kWalkCap) { *capped = 1; break; }
     float z = rnd_tea(seed);
-    hr = out ? sample_height(dist, wo, hr, z, ax, ay) : -sample_height(dist, -wo, -hr, z, ax, ay);
+    hr = sample_height(dist, out ? wo : -wo, out ? hr : -hr, z, ax, ay);
+    if (!out) hr = -hr;
     if (hr == kDefaultMax || hr == -kDefaultMax) break;
     order++;
     bool wi_out = out;
@@ -837,11 +887,12 @@ PT_D float ms_dielectric_eval(uint32_t dist, const float3& wi, const float3& wo,
     else { if (!(order == 0 || (uint32_t)cur <= order)) break; }
     if (it >= kWalkCap) { *capped = 1; break; }
     float z = rnd_tea(seed);
-    hr = wr_out ? sample_height(dist, wr, hr, z, ax, ay) : -sample_height(dist, -wr, -hr, z, ax, ay);
+    hr = sample_height(dist, wr_out ? wr : -wr, wr_out ? hr : -hr, z, ax, ay);
+    if (!wr_out) hr = -hr;
     if (hr == kDefaultMax || hr == -kDefaultMax || isinf(hr)) break;
     cur++;
     float phase = eval_dielectric_phase(dist, -wr, wo, wr_out, wo_out, eta, ax, ay);
-    float shadow = wo_out ? G_height(dist, wo, hr, ax, ay) : G_height(dist, -wo, -hr, ax, ay);
+    float shadow = G_height(dist, wo_out ? wo : -wo, wo_out ? hr : -hr, ax, ay);
     float I = phase * shadow;
     if (dist == GGX) sum += I;
     else if (isfinite(I) && (order == 0 || (uint32_t)cur == order)) sum += I;

@@ -11,7 +11,7 @@
 //            rough_transparent_shader.cu, arealight_shader.cu, constantbg.cu; continuing paths are
 //            appended to the next active queue and diffuse next-event estimation to the shadow queue
 //   shadow   any-hit through the same BVH; unoccluded contributions are added to the path radiance
-// (a chunk of few paths runs all of its bounces in one launch of path pools instead, pt_pool.cu)
+// (a chunk of few paths runs all of its bounces in one launch of path pools instead, pt_pool.cuh)
 // and finally `accumulate` folds the frames into the float4 running mean in frame order
 // (path_tracer.cu:64-68).
 //
@@ -1021,7 +1021,7 @@ __global__ void __launch_bounds__(kBlock) k_probe_gen(WfDev w, SssDev g, uint64_
         if (rough) microfacet(w_i);
         float cos_i = fmaxf(dot(w_i, nrm), 0.0f);
         if (cos_i > 0.0f) {
-          float att = scene_any(S, pos, w_i, S.integ.scene_epsilon, r) ? 0.0f : 1.0f;
+          float att = occluded(S, pos, w_i, S.integ.scene_epsilon, r) ? 0.0f : 1.0f;
           Le = Le * (att * cos_i / light_pdf);
         } else {
           Le = f3s(0.0f);

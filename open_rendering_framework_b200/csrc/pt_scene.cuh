@@ -840,6 +840,25 @@ template <class G> PT_HD bool trace_any(const G& S, const float3& o, const float
   return r > 0;
 }
 
+// Any hit over the wide BVH by one thread, its stack in local memory (vertex programs that need a light's
+// visibility before they go on).
+template <class G> PT_HD bool trace_any_wide(const G& S, const float3& o, const float3& d, float tmin, float tmax)
+{
+  uint2 ring[kRing4], spill[kSpill4];
+  Stack4 stk;
+  stack4_init(stk, ring, 1, spill);
+  const RayPre4 rp = ray_pre4(o, d, S.trav_scale);
+  for (int cur = 0; cur != kDone4;) {
+    if (cur < 0) {
+      if (leaf_any(S, (uint32_t)cur, o, d, tmin, tmax)) return true;
+      cur = stack4_next(stk, tmax, false);
+    } else {
+      cur = trav4_node_any(S, cur, rp, tmin, tmax, stk);
+    }
+  }
+  return false;
+}
+
 // ------------------------------------------------------------------ analytic emitters
 // Record k of SceneDev::ana: (position, radius), (disk normal, kind), (radiance, light index); the
 // kind is stored as int bits.  Hits are tested after the triangles, emitters in light order, and

@@ -1,6 +1,6 @@
 // The wavefront's device state and the vertices of a path: one function per material class, following the
 // reference's material programs, on the per-path records.  The wavefront's shading kernels (pt_render.cu)
-// and the path pools (pt_pool.cu) run the same functions, so both give a path the same arithmetic.
+// and the path pools (pt_pool.cuh) run the same functions, so both give a path the same arithmetic.
 #pragma once
 #include <utility>
 #include <vector>
@@ -141,6 +141,16 @@ __device__ __forceinline__ float3 shading_normal(const SceneDev& S, const int4& 
     n = normalize(ld3(__ldg(S.geo + prim)));
   }
   return normalize(n);
+}
+
+// Visibility for the vertex programs that trace a shadow ray of their own (one copy, out of line).  Over
+// the wide BVH where its box tests hold, as the shadow kernels: layered 301 x 203 x 6 with the
+// multiple-scattering model 3.72 to 2.55 ms a pass.
+static __device__ __noinline__ bool occluded(const SceneDev& S, float3 o, float3 d, float tmin, float tmax)
+{
+  const TravGeom g = trav_geom(S);
+  const bool hit = g.nodes4 && wide_ray(o, d, tmin, g.trav_scale) ? trace_any_wide(g, o, d, tmin, tmax) : trace_any(g, o, d, tmin, tmax);
+  return hit || (S.n_ana && ana_any(S, o, d, tmin, tmax));
 }
 
 // ------------------------------------------------------------------ lights (LightSampler.h)
@@ -496,7 +506,7 @@ __device__ __forceinline__ bool rough_diffuse_vertex(const SceneDev& S, const Wf
   eval_direct(S, hit_pos, ls, w_l, radiance, ldist, t, clamped);
   radiance = radiance / light_pdf;
   const float cos_theta_l = dot(ffnormal, w_l);
-  if (cos_theta_l > 0.0f && !scene_any(S, hit_pos, w_l, S.integ.scene_epsilon, ldist)) {
+  if (cos_theta_l > 0.0f && !occluded(S, hit_pos, w_l, S.integ.scene_epsilon, ldist)) {
     const float3 Li = radiance;  // V * radiance with V = 1
     float3 add;
     if (ms) {  // :126-139
@@ -946,7 +956,7 @@ static __device__ bool rough_translucent_vertex(const SceneDev& S, const WfDev& 
   light_radiance = light_radiance / light_pdf;
   const float cos_l = dot(ffnormal, w_l);
   if (!inside && cos_l > 0.0f) {
-    const float V = scene_any(S, hit_pos, w_l, S.integ.scene_epsilon, ldist) ? 0.0f : 1.0f;
+    const float V = occluded(S, hit_pos, w_l, S.integ.scene_epsilon, ldist) ? 0.0f : 1.0f;
     if (V > 0.0f) {
       const float3 Li = V * light_radiance;
       float3 add;
@@ -1207,7 +1217,7 @@ template <class K> inline int full_wave(K kernel)
   return grid;
 }
 
-// ------------------------------------------------------------------ kernels of large vertex programs (pt_pool.cu)
+// ------------------------------------------------------------------ path pools and large vertex programs (pt_pool.cu, pt_pool_all.cu)
 // All bounces of the paths in the queue w.q_in (at most n of them) by path pools.  `programs`: the vertex
 // programs the pass needs beside diffuse, conductor, dielectric, emitter and miss.
 // Up to how many paths a chunk runs through pools instead of the wavefront's launches.  A bounce of the
@@ -1223,6 +1233,7 @@ inline uint64_t pool_max_paths(bool translucent, bool multi) { return translucen
 enum PoolPrograms { POOL_BASIC = 0, POOL_TRANSLUCENT = 1 /* and smooth translucent objects */, POOL_ALL = 2 };
 pt_status launch_path_pools(const SceneDev& S0, const WfDev& w, uint64_t n, bool multi, bool adjoint, PoolPrograms programs, int refill,
                             cudaStream_t stream);
+pt_status launch_path_pools_all(const SceneDev& S0, const WfDev& w, uint64_t n, bool multi, bool adjoint, int refill, cudaStream_t stream);
 // The wavefront's layered and translucent shading, and the conductors and dielectrics of a pass that holds
 // the multiple-scattering model.
 void launch_shade_layered(const WfDev& w, bool adjoint, cudaStream_t stream);
