@@ -22,6 +22,41 @@ __device__ unsigned long long g_bsdf_capped = 0;
 // kPart 0: the whole query.  kPart 1 / 2: the Beckmann launch in two halves with smaller code each --
 // 1 samples the microfacet normal m and the direction wi (m parked in f, pdf, F), 2 evaluates f, pdf
 // and F from wo, wi and m.
+template <uint32_t kDist, int kPart>
+__device__ __forceinline__ void bsdf_query(uint64_t k, const float* __restrict__ wo_soa, const float* __restrict__ alpha, uint64_t n, uint64_t first,
+                                           float eta, float* __restrict__ wi_soa, float* __restrict__ f_out, float* __restrict__ pdf_out,
+                                           float* __restrict__ F_out)
+{
+  const float3 nrm = f3(0.0f, 0.0f, 1.0f);
+  float3 wo = f3(__ldg(wo_soa + k), __ldg(wo_soa + n + k), __ldg(wo_soa + 2 * n + k));
+  float a = __ldg(alpha + k);
+  float3 m, wi;
+  if constexpr (kPart != 2) {
+    uint64_t i = first + k;
+    uint32_t s = tea16((uint32_t)i, 0u);
+    float u1 = rnd_tea(s);
+    float u2 = rnd_tea(s);
+    int capped = 0;
+    m = sample_visible_normal(kDist, wo, nrm, a, a, u1, u2, &capped);
+    wi = reflect(-wo, m);
+    wi_soa[k] = wi.x;
+    wi_soa[n + k] = wi.y;
+    wi_soa[2 * n + k] = wi.z;
+    if (capped) atomicAdd(&g_bsdf_capped, 1ull);
+  } else {
+    m = f3(f_out[k], pdf_out[k], F_out[k]);
+    wi = f3(wi_soa[k], wi_soa[n + k], wi_soa[2 * n + k]);
+  }
+  if constexpr (kPart == 1) {
+    f_out[k] = m.x;
+    pdf_out[k] = m.y;
+    F_out[k] = m.z;
+  } else {
+    f_out[k] = walter_bsdf(kDist, wo, wi, nrm, a, eta);
+    pdf_out[k] = eval_visible_normal(kDist, wo, m, nrm, a, a) / (4.0f * fabsf(dot(wo, m)));
+    F_out[k] = fresnel_R(wo, m, eta);
+  }
+}
 template <uint32_t kDist, int kPart = 0>
 __global__ void __launch_bounds__(256) k_bsdf_queries(const float* __restrict__ wo_soa, const float* __restrict__ alpha, uint64_t n,
                                                       uint64_t k_begin, uint64_t k_end, uint64_t first, float eta,
@@ -37,38 +72,31 @@ __global__ void __launch_bounds__(256) k_bsdf_queries(const float* __restrict__ 
     asm volatile("griddepcontrol.wait;" ::: "memory");
   else
     asm volatile("griddepcontrol.launch_dependents;");
-  const float3 nrm = f3(0.0f, 0.0f, 1.0f);
   for (uint64_t k = k_begin + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; k < k_end; k += (uint64_t)gridDim.x * blockDim.x) {
-    float3 wo = f3(__ldg(wo_soa + k), __ldg(wo_soa + n + k), __ldg(wo_soa + 2 * n + k));
-    float a = __ldg(alpha + k);
-    float3 m, wi;
-    if constexpr (kPart != 2) {
-      uint64_t i = first + k;
-      uint32_t s = tea16((uint32_t)i, 0u);
-      float u1 = rnd_tea(s);
-      float u2 = rnd_tea(s);
-      int capped = 0;
-      m = sample_visible_normal(kDist, wo, nrm, a, a, u1, u2, &capped);
-      wi = reflect(-wo, m);
-      wi_soa[k] = wi.x;
-      wi_soa[n + k] = wi.y;
-      wi_soa[2 * n + k] = wi.z;
-      if (capped) atomicAdd(&g_bsdf_capped, 1ull);
-    } else {
-      m = f3(f_out[k], pdf_out[k], F_out[k]);
-      wi = f3(wi_soa[k], wi_soa[n + k], wi_soa[2 * n + k]);
-    }
-    if constexpr (kPart == 1) {
-      f_out[k] = m.x;
-      pdf_out[k] = m.y;
-      F_out[k] = m.z;
-    } else {
-      f_out[k] = walter_bsdf(kDist, wo, wi, nrm, a, eta);
-      pdf_out[k] = eval_visible_normal(kDist, wo, m, nrm, a, a) / (4.0f * fabsf(dot(wo, m)));
-      F_out[k] = fresnel_R(wo, m, eta);
-    }
+    bsdf_query<kDist, kPart>(k, wo_soa, alpha, n, first, eta, wi_soa, f_out, pdf_out, F_out);
   }
   if constexpr (kPart == 1) asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// A small batch in one launch: the first `ggx_blocks` blocks take the GGX queries, the others the Beckmann
+// queries, whole.  Up to kSmallBatch queries the chip is not full and a batch costs its launches and one
+// query's latency (a Beckmann query's Newton steps), so one launch of narrow blocks, spread over the SMs, is
+// best; above, the split launches' smaller code is.  us a batch, three launches / one: 1 query 14.8 / 11.0,
+// 4,099 18.5 / 16.4, 65,536 24.6 / 22.6, 262,144 40.9 / 39.5, 524,288 65.3 / 67.3, 2,097,152 226.5 / 231.4.
+constexpr uint64_t kSmallBatch = 1 << 18;
+constexpr int kSmallBlock = 64;  // 32 to 128: the same
+__global__ void __launch_bounds__(kSmallBlock) k_bsdf_queries_small(const float* __restrict__ wo_soa, const float* __restrict__ alpha, uint64_t n,
+                                                                    uint64_t n_ggx, uint32_t ggx_blocks, uint64_t first, float eta,
+                                                                    float* __restrict__ wi_soa, float* __restrict__ f_out,
+                                                                    float* __restrict__ pdf_out, float* __restrict__ F_out)
+{
+  if (blockIdx.x < ggx_blocks) {
+    const uint64_t k = blockIdx.x * (uint64_t)kSmallBlock + threadIdx.x;
+    if (k < n_ggx) bsdf_query<GGX, 0>(k, wo_soa, alpha, n, first, eta, wi_soa, f_out, pdf_out, F_out);
+  } else {
+    const uint64_t k = n_ggx + (blockIdx.x - ggx_blocks) * (uint64_t)kSmallBlock + threadIdx.x;
+    if (k < n) bsdf_query<BECKMANN, 0>(k, wo_soa, alpha, n, first, eta, wi_soa, f_out, pdf_out, F_out);
+  }
 }
 
 __global__ void k_rng_streams(int kind, uint32_t* seeds, uint64_t n, uint32_t draws, float* out)
@@ -137,6 +165,13 @@ pt_status pt_bsdf_queries(const float* d_wo_soa, const float* d_alpha, uint64_t 
   const uint64_t n_ggx = n_ggx_below <= first_index ? 0 : (n_ggx_below - first_index < n ? n_ggx_below - first_index : n);
   const int block = 256;
   cudaStream_t st = (cudaStream_t)stream;
+  if (n <= kSmallBatch) {
+    const uint32_t gb = (uint32_t)((n_ggx + kSmallBlock - 1) / kSmallBlock), bb = (uint32_t)((n - n_ggx + kSmallBlock - 1) / kSmallBlock);
+    k_bsdf_queries_small<<<gb + bb, kSmallBlock, 0, st>>>(d_wo_soa, d_alpha, n, n_ggx, gb, first_index, eta, d_wi_soa, d_f, d_pdf, d_F);
+    count_launch();
+    PT_CHECK_CUDA(cudaGetLastError(), "pt_bsdf_queries launch");
+    return PT_OK;
+  }
   if (n_ggx > 0) {
     k_bsdf_queries<GGX><<<grid_for(n_ggx, block, 8), block, 0, st>>>(d_wo_soa, d_alpha, n, 0, n_ggx, first_index, eta, d_wi_soa, d_f, d_pdf,
                                                                      d_F);
