@@ -69,6 +69,8 @@ std::vector<uint64_t> graph_key(const Context& E, const PassLayout& L, const std
                         E.wf2.rays.p, E.wf2.state.p, E.wf2.counters.p, E.wf2.path_item.p})
     k.push_back((uint64_t)(uintptr_t)p);
   k.push_back(E.wf.cap);
+  k.push_back(E.wf2.cap);
+  k.push_back(E.probes_beside ? 1 : 0);
   k.push_back((uint64_t)E.opt.extend_mode);
   k.push_back((uint64_t)E.opt.refill);
   k.push_back((uint64_t)E.opt.bin_items);

@@ -257,7 +257,8 @@ struct Context {
   cudaStream_t stream2 = nullptr, side2[2] = {nullptr, nullptr};
   cudaEvent_t ev2_fork = nullptr, ev2_join = nullptr, ev2_shade = nullptr, ev2_shadow = nullptr;
   cudaEvent_t ev_start = nullptr, ev_acc = nullptr, ev_end2 = nullptr;
-  bool pass_dual = false;  // the last pass ran two pipelines (its counters are in wf and wf2)
+  bool pass_dual = false;  // the last pass ran two pipelines, or probes beside paths (its counters are in wf and wf2)
+  bool probes_beside = false;  // the current pass may run its probe paths in wf2, beside the camera paths
   bool profile = false;
   std::vector<cudaEvent_t> prof_events;  // pairs around each extend and gather launch when profiling
   std::vector<int> prof_kind;            // PROF_EXTEND or PROF_GATHER per pair

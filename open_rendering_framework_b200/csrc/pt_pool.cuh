@@ -49,6 +49,11 @@ __device__ __forceinline__ void pool_trace(const SceneDev& S0, const WfDev& w, P
   const uint32_t n = nc + ns;
   TravGeom g = trav_geom(S0);
   const unsigned lane = threadIdx.x & 31;
+  // few rays: each warp takes its share of them and no more, since the lanes of a warp take turns between
+  // nodes and leaves (a 96 x 64 frame alone: 280 to 257 us)
+  constexpr uint32_t kWarpsOfBlock = kPoolBlock / 32;
+  const uint32_t lanes = min(32u, (n + kWarpsOfBlock - 1) / kWarpsOfBlock);
+  const unsigned mine = lanes >= 32u ? 0xffffffffu : (1u << lanes) - 1u;
   bool has = false, any = false, drained = false;
   uint32_t pid = 0, e = 0;
   float3 o = f3s(0.0f), d = f3s(0.0f);
@@ -61,14 +66,14 @@ __device__ __forceinline__ void pool_trace(const SceneDev& S0, const WfDev& w, P
   stack4_init(s4, sm.stk + threadIdx.x, kPoolBlock, spill4);
   int cur = kDone4;
   for (;;) {
-    const unsigned idle = __ballot_sync(0xffffffffu, !has);
-    if (!drained && (__popc(idle) >= refill || idle == 0xffffffffu)) {
+    const unsigned idle = __ballot_sync(0xffffffffu, !has) & mine;
+    if (!drained && (__popc(idle) >= refill || idle == mine)) {
       uint32_t base = 0;
       if (lane == 0) base = atomicAdd(&sm.fetch, (uint32_t)__popc(idle));
       base = __shfl_sync(0xffffffffu, base, 0);
       if (base + __popc(idle) >= n) drained = true;
       const uint32_t i = base + __popc(idle & lanemask_lt());
-      if (!has && i < n) {
+      if (!has && lane < lanes && i < n) {
         any = i >= nc;
         e = any ? i - nc : i;
         pid = any ? sm.shadow[e] : path[e];
@@ -268,9 +273,9 @@ static pt_status launch_pool(K kernel, const SceneDev& S0, const WfDev& w, uint6
     wave = sm_count() * std::max(1, blocks);
     cache.push_back({{key, dev}, wave});
   }
-  // every block takes an equal share of a small pass, in whole warps
+  // every block takes an equal share of a small pass
   const uint64_t per = (n + wave - 1) / wave;
-  const uint32_t share = (uint32_t)std::min<uint64_t>(pool_size(kProg), std::max<uint64_t>(32, (per + 31) / 32 * 32));
+  const uint32_t share = (uint32_t)std::min<uint64_t>(pool_size(kProg), std::max<uint64_t>(4, (per + 3) / 4 * 4));
   const int grid = (int)std::max<uint64_t>(1, std::min<uint64_t>(wave, (n + share - 1) / share));
   kernel<<<grid, pool_threads(kProg), smem, stream>>>(S0, w, refill, share);
   PT_CHECK_CUDA(cudaGetLastError(), "path pool launch");

@@ -1193,6 +1193,9 @@ __global__ void k_geo_normals(SceneDev S, float4* geo)
   }
 }
 
+// Probe paths of a chunk that may run beside its camera paths: 47 MB of wavefront at most.
+constexpr uint64_t kProbesBesideMax = 1ull << 18;
+
 static pt_status ensure_wavefront(Wavefront& wf, uint64_t cap)
 {
   if (wf.cap >= cap && wf.counters.p) return PT_OK;
@@ -1416,6 +1419,9 @@ pt_status pass_resources(Context& E, const PassLayout& L, const std::vector<Scen
 {
   pt_status st = ensure_wavefront(E.wf, L.cap_paths);
   if (st == PT_OK && L.dual) st = ensure_wavefront(E.wf2, L.cap_paths);
+  // a small pass's probe paths run beside its camera paths, in a wavefront of their own where memory allows
+  E.probes_beside = st == PT_OK && L.sss && E.opt.pool && E.opt.overlap && L.cap_probes > 0 && L.cap_probes <= kProbesBesideMax &&
+                    (E.opt.pool == 2 || L.cap_paths <= pool_max_paths(true, scenes.size() > 1)) && ensure_wavefront(E.wf2, L.cap_probes) == PT_OK;
   if (st == PT_OK && L.sss) st = ensure_sss(E, E.wf.cap, L.g_slots, L.cap_probes, L.cap_sets);
   if (st == PT_OK) st = E.d_scene_tab.reserve(scenes.size() * sizeof(SceneDev), "scene table");
   if (st == PT_OK) st = E.d_item_tab.reserve(std::max<size_t>(L.items.size(), 1) * sizeof(ItemDev), "item table");
@@ -1427,7 +1433,7 @@ pt_status pass_resources(Context& E, const PassLayout& L, const std::vector<Scen
     if (!sd) PT_CHECK_CUDA(cudaStreamCreateWithFlags(&sd, cudaStreamNonBlocking), "side stream");
   for (cudaEvent_t* ev : {&E.ev_fork, &E.ev_join, &E.ev_shade, &E.ev_shadow})
     if (!*ev) PT_CHECK_CUDA(cudaEventCreateWithFlags(ev, cudaEventDisableTiming), "stream event");
-  if (L.dual) {
+  if (L.dual || E.probes_beside) {
     for (cudaStream_t* sd : {&E.stream2, &E.side2[0], &E.side2[1]})
       if (!*sd) PT_CHECK_CUDA(cudaStreamCreateWithFlags(sd, cudaStreamNonBlocking), "second pipeline stream");
     for (cudaEvent_t* ev : {&E.ev2_fork, &E.ev2_join, &E.ev2_shade, &E.ev2_shadow, &E.ev_start, &E.ev_acc, &E.ev_end2})
@@ -1491,7 +1497,7 @@ pt_status launch_pass(Context& E, const PassLayout& L, const std::vector<SceneDe
   Wavefront* const wf_of[2] = {&c.wf, dual ? &c.wf2 : &c.wf};
   WfDev w = w_of[0];
   Wavefront* wf = wf_of[0];
-  c.pass_dual = dual;
+  c.pass_dual = dual || c.probes_beside;
   Wavefront& wf0 = c.wf;
   SssDev g;
   memset(&g, 0, sizeof(g));
@@ -1531,6 +1537,7 @@ pt_status launch_pass(Context& E, const PassLayout& L, const std::vector<SceneDe
     PT_CHECK_CUDA(cudaStreamWaitEvent(c.stream2, c.ev_start, 0), "second pipeline start");
     PT_CHECK_CUDA(cudaMemsetAsync(w_of[1].cnt, 0, kCounters * 4, c.stream2), "reset counters");
   }
+  if (c.probes_beside) PT_CHECK_CUDA(cudaMemsetAsync(c.wf2.counters.p, 0, kCounters * 4, c.stream), "reset counters");
   c.prof_pairs = 0;
   pt_status st = PT_OK;
   // CUDA events around the launches whose device time the stats report (when profiling is on)
@@ -1580,11 +1587,15 @@ pt_status launch_pass(Context& E, const PassLayout& L, const std::vector<SceneDe
     PT_CHECK_CUDA(cudaStreamWaitEvent(waiter, ev, 0), "stream fork / join");
     return PT_OK;
   };
+  // a chunk of n paths runs its bounces by path pools
+  auto by_pools = [&](uint64_t n) {
+    return c.opt.pool && !prof && w4 && c.opt.extend_mode == 1 && (c.opt.pool == 2 || n <= pool_max_paths(L.sss, multi));
+  };
+  const PoolPrograms programs = L.ms || L.layered || L.rough ? POOL_ALL : L.sss ? POOL_TRANSLUCENT : POOL_BASIC;
   // L.passes = max_depth + 2 bounces: every path has ended by then (each shader stops at max_depth).
   auto bounces = [&](uint64_t n, bool adj_pass) -> pt_status {
     const bool adjoint = adj_pass;
-    if (c.opt.pool && !prof && w4 && c.opt.extend_mode == 1 && (c.opt.pool == 2 || n <= pool_max_paths(L.sss, multi))) {
-      const PoolPrograms programs = L.ms || L.layered || L.rough ? POOL_ALL : L.sss ? POOL_TRANSLUCENT : POOL_BASIC;
+    if (by_pools(n)) {
       if ((st = launch_path_pools(S0, w, n, multi, adjoint, programs, c.opt.refill, s_main)) != PT_OK) return st;
       count_launch();
       ++c.stats.extend_launches;
@@ -1698,7 +1709,30 @@ pt_status launch_pass(Context& E, const PassLayout& L, const std::vector<SceneDe
     S0 = tab[w.scene0];
     grid_persist = grid_persist_of[multi ? 1 : 0];
     const uint64_t n_paths = L.chunk_paths[k], n_probes = L.chunk_probes[k];
-    if (n_probes) {
+    // the camera paths do not read the probes (their gathers are evaluated at the end), so where both are
+    // small the probe pass runs on a stream and in a wavefront of its own until the gathers
+    const bool beside = n_probes && c.probes_beside && n_probes <= c.wf2.cap && by_pools(n_paths) && by_pools(n_probes);
+    if (beside) {
+      WfDev p = make_w(c.wf2);
+      p.items = w.items;
+      p.n_items = w.n_items;
+      p.multi = w.multi;
+      p.scene0 = w.scene0;
+      p.adj_a = p.adj_b = nullptr;
+      p.q_in = c.wf2.q_a.as<uint32_t>();
+      p.q_out = c.wf2.q_b.as<uint32_t>();
+      p.in_slot = CNT_ACTIVE_A;
+      p.out_slot = CNT_ACTIVE_B;
+      PT_CHECK_CUDA(cudaEventRecord(c.ev_start, s_main), "probe pass start");
+      PT_CHECK_CUDA(cudaStreamWaitEvent(c.stream2, c.ev_start, 0), "probe pass start");
+      PT_CHECK_CUDA(cudaMemsetAsync(p.cnt, 0, (CNT_FETCH_SH + 1) * 4, c.stream2), "reset queues");
+      k_probe_gen<<<grid_for(n_probes, kBlock, 16), kBlock, 0, c.stream2>>>(p, g, 0, n_probes);
+      if ((st = launch_path_pools(S0, p, n_probes, multi, false, programs, c.opt.refill, c.stream2)) != PT_OK) return st;
+      k_probe_finish<<<grid_for(n_probes, kBlock, 16), kBlock, 0, c.stream2>>>(p, g, 0, n_probes);
+      k_probe_compact<<<L.chunk_sets[k], 256, 0, c.stream2>>>(p, g);
+      count_launch(4);
+      PT_CHECK_CUDA(cudaEventRecord(c.ev_end2, c.stream2), "probe pass join");
+    } else if (n_probes) {
       for (uint64_t j0 = 0; j0 < n_probes; j0 += w.cap) {
         uint64_t nj = std::min<uint64_t>(w.cap, n_probes - j0);
         if ((st = reset_queues()) != PT_OK) return st;
@@ -1717,6 +1751,7 @@ pt_status launch_pass(Context& E, const PassLayout& L, const std::vector<SceneDe
     count_launch();
     if ((st = bounces(n_paths, adjoint)) != PT_OK) return st;
     if (n_probes) {
+      if (beside) PT_CHECK_CUDA(cudaStreamWaitEvent(s_main, c.ev_end2, 0), "probe pass join");
       PT_CHECK_CUDA(cudaMemsetAsync(w.cnt + CNT_GATHER, 0, 8, s_main), "reset gather list");
       uint32_t* list = wf->q_a.as<uint32_t>();
       k_gather_collect<<<grid_for(n_paths, kBlock, 16), kBlock, 0, s_main>>>(w, n_paths, list);

@@ -94,3 +94,22 @@ def test_pool_option_rejects_other_values(value):
     with pytest.raises(Exception):
         R.set_option("pool", value)
     R.close()
+
+
+@pytest.mark.parametrize("probes,frames", [(1, 1), (70, 3), (3000, 2)])
+def test_probe_paths_beside_the_camera_paths(probes, frames):
+    """The probe pass on its own stream and wavefront (option overlap 1, pools) against the one after the other
+    (overlap 0) and the wavefront's launches (pool 0): images, counters and probe records are identical, over
+    two renders of one context."""
+    got = []
+    for pool, overlap in ((1, 1), (1, 0), (0, 1)):
+        R = sc.Renderer(scenes.translucent_box_scene(40, 31, probe_samples=probes, two_objects=True))
+        R.set_option("pool", pool)
+        R.set_option("overlap", overlap)
+        R.render(frames)
+        first = [getattr(R.stats(), k) for k in COUNTS]
+        R.render(frames)
+        got.append((R.readback().view(np.uint32), first, [getattr(R.stats(), k) for k in COUNTS], R.probes().tobytes()))
+        R.close()
+    for other in got[1:]:
+        assert np.array_equal(got[0][0], other[0]) and got[0][1:] == other[1:]
