@@ -661,7 +661,8 @@ __global__ void __launch_bounds__(kBlock) k_gather_collect(WfDev w, uint64_t n_p
 // One thread per path with the exact test in the probe loop and the dipole on the accepting lanes took
 // 19.6 ms for 456,028 gathers of 3,011 pairs (512 x 512 x 4 frames, 4,096 probes: 69.9 Gpair/s); this
 // takes 16.2 ms (84.8).  Gathers of few pairs and many acceptances (175,143 of 312 pairs, scale 10): 3.04
-// to 1.27 ms.  Five blocks per SM: with 6 to 8 the evaluation spills and the times are the same or worse.
+// to 1.27 ms.  Six blocks per SM with the evaluation out of line: 5 blocks the same, 8 to 12 spill and are 2 to
+// 4 % slower.
 //
 // A differentiable forward render also stores each gather's value with the path (adj_G).  kAdj: the
 // adjoint replays the same chain; a queued pair of a differentiated material adds the standard dipole's
@@ -712,6 +713,58 @@ __device__ __forceinline__ void gather_grad_emit(GatherGrad& a, int lane)
   }
 }
 
+// One queued pair of the warp: its value (forward: the term with its weight; adjoint: d / d sigma_a and
+// d / d sigma_s') where the exact test accepts it.  Out of line, so that the probe loop keeps its registers.
+struct GatherValue {
+  float3 v, ds;
+  int ok;
+};
+template <bool kAdj>
+static __device__ __noinline__ GatherValue gather_eval(const SceneDev* scenes, const float4* pc_pos, const float4* pc_wl, const float4* pc_nrm,
+                                                       const float4* pc_tr, const GatherWarp* sp, int lane)
+{
+  const GatherWarp& s = *sp;
+  GatherValue r{f3s(0.0f), f3s(0.0f), 0};
+  const uint4 e = s.q[lane];
+  const uint32_t o = e.x;
+  const float4 x4 = s.xo[o], f4 = s.f[o];
+  const uint2 id = s.sm[o];
+  const SceneDev& S = scenes[id.x];
+  const ScatDev& P = S.scat[id.y];
+  const uint64_t at = s.pb[o] + e.y;
+  const float3 xo = ld3(x4);
+  const float3 pos = ld3(__ldg(pc_pos + at));
+  const float dist = length(xo - pos);
+  const float exp_term = expf(-dist * x4.w);
+  const float rn = md5_draw(e.z, e.w);
+  if constexpr (kAdj) {
+    if (rn < exp_term) {
+      const float scale = S.mats[id.y].a.x;
+      const float3 wl = ld3(__ldg(pc_wl + at));
+      const Dual2 sx = dipole_channel_grad(dist, P.absorption.x, P.reducedExtinction.x, P.A.x, scale);
+      const Dual2 sy = dipole_channel_grad(dist, P.absorption.y, P.reducedExtinction.y, P.A.y, scale);
+      const Dual2 sz = dipole_channel_grad(dist, P.absorption.z, P.reducedExtinction.z, P.A.z, scale);
+      const float3 k = ld3(f4) * wl / exp_term;
+      r.v = k * f3(sx.da, sy.da, sz.da);
+      r.ds = k * f3(sx.ds, sy.ds, sz.ds);
+      r.ok = 1;
+    }
+  } else {
+    const bool rough = f4.w != 0.0f;  // rough boundary: draws must exceed 0.001, terms carry the weight
+    if (rn < exp_term && (!rough || rn > 0.001f)) {
+      const float3 wl = ld3(__ldg(pc_wl + at));
+      float3 term;
+      if (S.mats[id.y].model == DIRECTIONAL_DIPOLE)
+        term = wl * dirpole_bssrdf(pos, ld3(__ldg(pc_nrm + at)), ld3(__ldg(pc_tr + at)), xo, ld3(s.no[o]), P) / exp_term;
+      else
+        term = wl * dipole_bssrdf(dist, std_dipole_terms(P)) / exp_term;
+      r.v = rough ? term * ld3(f4) : term;
+      r.ok = 1;
+    }
+  }
+  return r;
+}
+
 // Evaluates the first `count` queued pairs of the warp, one per lane.  Forward: adds the values of the
 // calling lane's own pairs (bits of `mine`, queue order = probe order) to acc.  Adjoint: adds the pair's
 // derivatives to grad.
@@ -720,50 +773,15 @@ __device__ __forceinline__ void gather_flush(const WfDev& w, const SssDev& g, Ga
                                              GatherGrad& grad)
 {
   __syncwarp();
-  float3 v = f3s(0.0f), ds = f3s(0.0f);
-  float* gr = nullptr;
-  bool ok = false;
-  if (lane < count) {
-    const uint4 e = s.q[lane];
-    const uint32_t o = e.x;
-    const float4 x4 = s.xo[o], f4 = s.f[o];
-    const uint2 id = s.sm[o];
-    const SceneDev& S = w.scenes[id.x];
-    const ScatDev& P = S.scat[id.y];
-    const uint64_t at = s.pb[o] + e.y;
-    const float3 xo = ld3(x4);
-    const float3 pos = ld3(__ldg(g.pc_pos + at));
-    const float dist = length(xo - pos);
-    const float exp_term = expf(-dist * x4.w);
-    const float rn = md5_draw(e.z, e.w);
-    if constexpr (kAdj) {
-      ok = rn < exp_term;
-      if (ok) {
-        const float scale = S.mats[id.y].a.x;
-        gr = S.mat_grad[id.y];
-        const float3 wl = ld3(__ldg(g.pc_wl + at));
-        const Dual2 sx = dipole_channel_grad(dist, P.absorption.x, P.reducedExtinction.x, P.A.x, scale);
-        const Dual2 sy = dipole_channel_grad(dist, P.absorption.y, P.reducedExtinction.y, P.A.y, scale);
-        const Dual2 sz = dipole_channel_grad(dist, P.absorption.z, P.reducedExtinction.z, P.A.z, scale);
-        const float3 k = ld3(f4) * wl / exp_term;
-        v = k * f3(sx.da, sy.da, sz.da);
-        ds = k * f3(sx.ds, sy.ds, sz.ds);
-      }
-    } else {
-      const bool rough = f4.w != 0.0f;  // rough boundary: draws must exceed 0.001, terms carry the weight
-      ok = rn < exp_term && (!rough || rn > 0.001f);
-      if (ok) {
-        const float3 wl = ld3(__ldg(g.pc_wl + at));
-        float3 term;
-        if (S.mats[id.y].model == DIRECTIONAL_DIPOLE)
-          term = wl * dirpole_bssrdf(pos, ld3(__ldg(g.pc_nrm + at)), ld3(__ldg(g.pc_tr + at)), xo, ld3(s.no[o]), P) / exp_term;
-        else
-          term = wl * dipole_bssrdf(dist, std_dipole_terms(P)) / exp_term;
-        v = rough ? term * ld3(f4) : term;
-      }
-    }
-  }
+  GatherValue e{f3s(0.0f), f3s(0.0f), 0};
+  if (lane < count) e = gather_eval<kAdj>(w.scenes, g.pc_pos, g.pc_wl, g.pc_nrm, g.pc_tr, &s, lane);
+  __syncwarp();
   if constexpr (kAdj) {
+    float* gr = nullptr;
+    if (e.ok) {
+      const uint2 id = s.sm[s.q[lane].x];
+      gr = w.scenes[id.x].mat_grad[id.y];
+    }
     const unsigned have = __ballot_sync(0xffffffffu, gr != nullptr);
     if (have == 0) return;
     const unsigned long long g0 = __shfl_sync(0xffffffffu, (unsigned long long)gr, __ffs(have) - 1);
@@ -772,22 +790,22 @@ __device__ __forceinline__ void gather_flush(const WfDev& w, const SssDev& g, Ga
         gather_grad_emit(grad, lane);
         grad.g = (float*)g0;
       }
-      grad.v[0] += v.x;
-      grad.v[1] += v.y;
-      grad.v[2] += v.z;
-      grad.v[3] += ds.x;
-      grad.v[4] += ds.y;
-      grad.v[5] += ds.z;
+      grad.v[0] += e.v.x;
+      grad.v[1] += e.v.y;
+      grad.v[2] += e.v.z;
+      grad.v[3] += e.ds.x;
+      grad.v[4] += e.ds.y;
+      grad.v[5] += e.ds.z;
     } else if (gr) {
-      atomicAdd(gr + 0, v.x);
-      atomicAdd(gr + 1, v.y);
-      atomicAdd(gr + 2, v.z);
-      atomicAdd(gr + 3, ds.x);
-      atomicAdd(gr + 4, ds.y);
-      atomicAdd(gr + 5, ds.z);
+      atomicAdd(gr + 0, e.v.x);
+      atomicAdd(gr + 1, e.v.y);
+      atomicAdd(gr + 2, e.v.z);
+      atomicAdd(gr + 3, e.ds.x);
+      atomicAdd(gr + 4, e.ds.y);
+      atomicAdd(gr + 5, e.ds.z);
     }
   } else {
-    s.val[lane] = make_float4(v.x, v.y, v.z, ok ? 1.0f : 0.0f);
+    s.val[lane] = make_float4(e.v.x, e.v.y, e.v.z, e.ok ? 1.0f : 0.0f);
     __syncwarp();
     for (; mine; mine &= mine - 1) {
       const float4 t = s.val[__ffs(mine) - 1];
@@ -797,7 +815,7 @@ __device__ __forceinline__ void gather_flush(const WfDev& w, const SssDev& g, Ga
 }
 
 template <bool kAdj>
-__global__ void __launch_bounds__(kBlock, 5) k_gather(WfDev w, SssDev g, const uint32_t* list, uint32_t one)
+__global__ void __launch_bounds__(kBlock, 6) k_gather(WfDev w, SssDev g, const uint32_t* list, uint32_t one)
 {
   __shared__ GatherWarp shared[kWarps];
   const uint32_t n = w.cnt[CNT_GATHER];
