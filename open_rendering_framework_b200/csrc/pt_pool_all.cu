@@ -29,7 +29,7 @@ __global__ void __launch_bounds__(kBlock) k_shade_layered(WfDev w)
     NeeRay nee;
     if (i < n) {
       pid = q[i];
-      cont = layered_path<kAdj>(w, pid, nee, shadow, clamped, overflow, capped_total);
+      cont = layered_path<kAdj>(scene_of(w, pid), w, pid, nee, shadow, clamped, overflow, capped_total);
     }
     const uint32_t s_slot = block_slot(shadow, w.cnt + CNT_SHADOW, sm);
     if (shadow) {
@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(kBlock) k_shade_translucent(WfDev w)
     uint32_t pid = 0;
     if (i < n) {
       pid = q[i];
-      cont = translucent_path<kAdj, kRough>(w, pid, overflow, clamped, capped);
+      cont = translucent_path<kAdj, kRough>(scene_of(w, pid), w, pid, overflow, clamped, capped);
     }
     uint32_t c_slot = block_slot(cont, w.cnt + w.out_slot, sm);
     if (cont) w.q_out[c_slot] = pid;

@@ -574,7 +574,7 @@ __global__ void __launch_bounds__(kBlock) k_shade_miss(WfDev w)
   const uint32_t* q = w.q_mat + (size_t)QC_MISS * w.cap;
   for (uint32_t i = blockIdx.x * kBlock + threadIdx.x; i < n; i += gridDim.x * kBlock) {
     uint32_t pid = q[i];
-    miss_path<kAdj>(w, pid);
+    miss_path<kAdj>(scene_of(w, pid), w, pid);
   }
 }
 
@@ -585,7 +585,7 @@ __global__ void __launch_bounds__(kBlock) k_shade_light(WfDev w)
   const uint32_t* q = w.q_mat + (size_t)QC_LIGHT * w.cap;
   for (uint32_t i = blockIdx.x * kBlock + threadIdx.x; i < n; i += gridDim.x * kBlock) {
     uint32_t pid = q[i];
-    light_path<kAdj>(w, pid);
+    light_path<kAdj>(scene_of(w, pid), w, pid);
   }
 }
 
@@ -604,7 +604,7 @@ __global__ void __launch_bounds__(kBlock) k_shade_diffuse(WfDev w)
     NeeRay nee;
     if (i < n) {
       pid = q[i];
-      cont = diffuse_path<kAdj>(w, pid, nee, shadow, clamped, overflow);
+      cont = diffuse_path<kAdj>(scene_of(w, pid), w, pid, nee, shadow, clamped, overflow);
     }
     uint32_t s_slot = block_slot(shadow, w.cnt + CNT_SHADOW, sm);
     if (shadow) {
@@ -617,8 +617,6 @@ __global__ void __launch_bounds__(kBlock) k_shade_diffuse(WfDev w)
   if (clamped) atomicAdd(cnt64(w.cnt, CNT_CLAMPED), (unsigned long long)clamped);
   if (overflow) atomicAdd(cnt64(w.cnt, CNT_ERROR), (unsigned long long)overflow);
 }
-
-
 
 // Paths with pending dipole gathers, appended to `out` (warp-aggregated).
 __global__ void __launch_bounds__(kBlock) k_gather_collect(WfDev w, uint64_t n_paths, uint32_t* out)

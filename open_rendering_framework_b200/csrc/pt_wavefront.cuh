@@ -430,9 +430,8 @@ __device__ __forceinline__ void put_nee(const WfDev& w, uint32_t at, const NeeRa
 // kAdj (all shade kernels): the adjoint replay; the first thing done for a path is adding the pending
 // gradient of its previous vertex, and what the forward adds to the path radiance is taken off R.
 template <bool kAdj>
-__device__ __forceinline__ void miss_path(const WfDev& w, uint32_t pid)
+__device__ __forceinline__ void miss_path(const SceneDev& S, const WfDev& w, uint32_t pid)
 {
-  const SceneDev& S = scene_of(w, pid);
   if constexpr (kAdj) apply_pending(S, w, pid);
   float3 bg = S.bg_color;
   if (S.env.present) {
@@ -446,9 +445,8 @@ __device__ __forceinline__ void miss_path(const WfDev& w, uint32_t pid)
 
 // arealight_shader.cu:36-50: emitted radiance if the hit is front-facing and emission is enabled.
 template <bool kAdj>
-__device__ __forceinline__ void light_path(const WfDev& w, uint32_t pid)
+__device__ __forceinline__ void light_path(const SceneDev& S, const WfDev& w, uint32_t pid)
 {
-  const SceneDev& S = scene_of(w, pid);
   if constexpr (kAdj) apply_pending(S, w, pid);
   if (!(w.rng[pid].w & META_EMIT)) return;
   float4 h = w.hit[pid], d = w.ray_d[pid];
@@ -577,10 +575,9 @@ __device__ __forceinline__ bool rough_diffuse_vertex(const SceneDev& S, const Wf
 // Neither is differentiable (pt_render_adjoint rejects them); the adjoint variant only settles the
 // pending gradient of the previous vertex and replays the path.
 template <bool kAdj>
-__device__ __forceinline__ bool layered_path(const WfDev& w, uint32_t pid, NeeRay& nee, bool& shadow, uint32_t& clamped, uint32_t& overflow, uint32_t& capped_total)
+__device__ __forceinline__ bool layered_path(const SceneDev& S, const WfDev& w, uint32_t pid, NeeRay& nee, bool& shadow, uint32_t& clamped, uint32_t& overflow, uint32_t& capped_total)
 {
   bool cont = false;
-  const SceneDev& S = scene_of(w, pid);
   if constexpr (kAdj) apply_pending(S, w, pid);
   nee.eps = S.integ.scene_epsilon;
   const uint4 rg = w.rng[pid];
@@ -648,10 +645,9 @@ __device__ __forceinline__ bool layered_path(const WfDev& w, uint32_t pid, NeeRa
 // diffuse_shader.cu:42-107.  Adjoint: an albedo texel's gradient through the next-event estimate
 // (resolved with the shadow ray) and through the bounce weight albedo / p (pending).
 template <bool kAdj>
-__device__ __forceinline__ bool diffuse_path(const WfDev& w, uint32_t pid, NeeRay& nee, bool& shadow, uint32_t& clamped, uint32_t& overflow)
+__device__ __forceinline__ bool diffuse_path(const SceneDev& S, const WfDev& w, uint32_t pid, NeeRay& nee, bool& shadow, uint32_t& clamped, uint32_t& overflow)
 {
   bool cont = false;
-  const SceneDev& S = scene_of(w, pid);
   if constexpr (kAdj) apply_pending(S, w, pid);
   nee.eps = S.integ.scene_epsilon;
   // the path's records are loaded before the depth test (every queued id has them), so that their
@@ -723,10 +719,9 @@ __device__ __forceinline__ bool diffuse_path(const WfDev& w, uint32_t pid, NeeRa
 // kMS: some conductor of the pass uses the multiple-scattering model (else that code is left out,
 // which keeps the kernel's instruction footprint small).
 template <bool kAdj, bool kMS>
-__device__ __forceinline__ bool metal_path(const WfDev& w, uint32_t pid, uint32_t& capped_total, uint32_t& overflow)
+__device__ __forceinline__ bool metal_path(const SceneDev& S, const WfDev& w, uint32_t pid, uint32_t& capped_total, uint32_t& overflow)
 {
   bool cont = false;
-  const SceneDev& S = scene_of(w, pid);
   if constexpr (kAdj) apply_pending(S, w, pid);
   uint4 rg = w.rng[pid];
   float4 h = w.hit[pid], o = w.ray_o[pid], d4 = w.ray_d[pid];
@@ -830,10 +825,9 @@ __device__ __forceinline__ DirSeed smooth_glass_dir(float3 d, float3 normal, flo
 // previous vertex.
 // kMS: some rough dielectric of the pass uses the multiple-scattering model (as for k_shade_metal).
 template <bool kAdj, bool kMS>
-__device__ __forceinline__ bool glass_path(const WfDev& w, uint32_t pid, uint32_t& capped_total, uint32_t& overflow)
+__device__ __forceinline__ bool glass_path(const SceneDev& S, const WfDev& w, uint32_t pid, uint32_t& capped_total, uint32_t& overflow)
 {
   bool cont = false;
-  const SceneDev& S = scene_of(w, pid);
   if constexpr (kAdj) apply_pending(S, w, pid);
   uint4 rg = w.rng[pid];
   float4 h = w.hit[pid], o = w.ray_o[pid], d4 = w.ray_d[pid];
@@ -1067,10 +1061,9 @@ static __device__ bool rough_translucent_vertex(const SceneDev& S, const WfDev& 
 // was stored with the path); its gradient is added at the end (k_gather<true>).  Inside, the weight
 // beam_T / p has p detached: d w / d sigma_a / w = -t * scale per channel.
 template <bool kAdj, bool kRough>
-__device__ __forceinline__ bool translucent_path(const WfDev& w, uint32_t pid, uint32_t& overflow, uint32_t& clamped, int& capped)
+__device__ __forceinline__ bool translucent_path(const SceneDev& S, const WfDev& w, uint32_t pid, uint32_t& overflow, uint32_t& clamped, int& capped)
 {
   bool cont = false;
-  const SceneDev& S = scene_of(w, pid);
   if constexpr (kAdj) apply_pending(S, w, pid);
   uint4 rg = w.rng[pid];
   float4 h = w.hit[pid], o = w.ray_o[pid], d4 = w.ray_d[pid];
@@ -1171,7 +1164,7 @@ __global__ void __launch_bounds__(kBlock) k_shade_metal(WfDev w)
     uint32_t pid = 0;
     if (i < n) {
       pid = q[i];
-      cont = metal_path<kAdj, kMS>(w, pid, capped_total, overflow);
+      cont = metal_path<kAdj, kMS>(scene_of(w, pid), w, pid, capped_total, overflow);
     }
     uint32_t c_slot = block_slot(cont, w.cnt + w.out_slot, sm);
     if (cont) w.q_out[c_slot] = pid;
@@ -1193,7 +1186,7 @@ __global__ void __launch_bounds__(kBlock) k_shade_glass(WfDev w)
     uint32_t pid = 0;
     if (i < n) {
       pid = q[i];
-      cont = glass_path<kAdj, kMS>(w, pid, capped_total, overflow);
+      cont = glass_path<kAdj, kMS>(scene_of(w, pid), w, pid, capped_total, overflow);
     }
     uint32_t c_slot = block_slot(cont, w.cnt + w.out_slot, sm);
     if (cont) w.q_out[c_slot] = pid;
