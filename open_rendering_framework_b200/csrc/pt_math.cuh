@@ -78,9 +78,10 @@ PT_HD uint32_t tea16(uint32_t v0, uint32_t v1)
 // height sampler and masking -- where inlined copies overflow the instruction cache.
 //
 // tea_hash / rnd_tea, random.h:117-127 (the draw may round up to exactly 1.0f).
-#ifdef PT_OUTLINE_TEA
+#if defined(PT_OUTLINE_TEA) || defined(PT_OUTLINE_TEA_BECKMANN)
 static __device__ __noinline__ uint32_t tea_call(uint32_t v) { return tea16(v, 100u); }
 #endif
+PT_HD float tea_float(uint32_t s) { return (float)(s & 0x7FFFFFFFu) / (float)0x80000000u; }
 PT_HD float rnd_tea(uint32_t& prev)
 {
 #if defined(PT_OUTLINE_TEA) && defined(__CUDA_ARCH__)
@@ -88,7 +89,7 @@ PT_HD float rnd_tea(uint32_t& prev)
 #else
   prev = tea16(prev, 100u);
 #endif
-  return (float)(prev & 0x7FFFFFFFu) / (float)0x80000000u;
+  return tea_float(prev);
 }
 // lcg / rnd, random.h:43-61.
 PT_HD float rnd_lcg(uint32_t& prev)
@@ -592,6 +593,9 @@ PT_D float2 bk_P22(float theta_i, float z1, float z2, int* capped)
   float emax = fmaxf(emin, erff(slope_i));
   float ecur = 0.5f * (emin + emax);
   int it = 0;
+  // the loop mostly ends at a point whose slope it has just taken (|cdf - z1| < 1e-5, ecur in [emin, emax])
+  bool have = false;
+  float slope = 0.0f;
   while (emax - emin > 0.00001f) {
     if (++it > kNewtonCap) { *capped = 1; break; }
     if (!(ecur >= emin && ecur <= emax)) ecur = 0.5f * (emin + emax);
@@ -604,7 +608,11 @@ PT_D float2 bk_P22(float theta_i, float z1, float z2, int* capped)
       cdf = (float)((double)c * inner);
     }
     float diff = cdf - z1;
-    if (fabsf(diff) < 0.00001f) break;
+    if (fabsf(diff) < 0.00001f) {
+      have = true;
+      slope = sv;
+      break;
+    }
     if (diff > 0.0f) {
       if (emax == ecur) break;
       emax = ecur;
@@ -615,7 +623,8 @@ PT_D float2 bk_P22(float theta_i, float z1, float z2, int* capped)
     float deriv = 0.5f * c * cos_i - 0.5f * c * sin_i * sv;
     ecur -= diff / deriv;
   }
-  return make_float2((float)erfinv_giles((double)fminf(emax, fmaxf(emin, ecur))), (float)erfinv_giles((double)(2.0f * z2 - 1.0f)));
+  if (!have) slope = (float)erfinv_giles((double)fminf(emax, fmaxf(emin, ecur)));
+  return make_float2(slope, (float)erfinv_giles((double)(2.0f * z2 - 1.0f)));
 }
 PT_D float bk_eval_ndf(const float3& wm, float ax, float ay)  // :249-261 with :61-65
 {
@@ -733,6 +742,19 @@ PT_D float walter_bsdf(uint32_t dist, const float3& wi, const float3& wo, const 
 }
 
 // ------------------------------------------------------------------ multiscattering walks
+// A walk's draw.  PT_OUTLINE_TEA_BECKMANN: the translation unit's Beckmann walks call one copy (their code
+// overflows the instruction cache: evaluating the diffuse walk 667 to 571 us for 500,009 queries); the GGX
+// walks, which are shorter, keep it inlined (called, they lose 3 to 5 %).
+PT_D float walk_draw(uint32_t dist, uint32_t& seed)
+{
+#if defined(PT_OUTLINE_TEA_BECKMANN)
+  if (dist != GGX) {
+    seed = tea_call(seed);
+    return tea_float(seed);
+  }
+#endif
+  return rnd_tea(seed);
+}
 PT_D float sample_height_inline(uint32_t dist, const float3& wr, float hr, float z, float ax, float ay)
 {
   if (dist == GGX) {  // MicrofacetGGX.h:254-276
@@ -774,7 +796,7 @@ PT_D float G_height(uint32_t dist, const float3& wi, float h, float ax, float ay
 PT_D float3 sample_dielectric_phase(uint32_t dist, const float3& wi, float3& wm, float m_eta, uint32_t& seed, bool wi_out,
                                     bool& wo_out, float ax, float ay, int* capped)
 {
-  float z1 = rnd_tea(seed), z2 = rnd_tea(seed);
+  float z1 = walk_draw(dist, seed), z2 = walk_draw(dist, seed);
   float eta = wi_out ? m_eta : 1.0f / m_eta;
   wm = sample_vndf(dist, wi_out ? wi : -wi, ax, ay, z1, z2, capped);
   if (!wi_out) wm = -wm;
@@ -782,7 +804,7 @@ PT_D float3 sample_dielectric_phase(uint32_t dist, const float3& wi, float3& wm,
   float st2 = eta * eta * (1.0f - ct * ct);
   float ctt = sqrtf(1.0f - st2);
   float F = st2 < 1.0f ? fresnel_R(ct, ctt, eta) : 1.0f;
-  if (rnd_tea(seed) <= F) return normalize(-wi + 2.0f * wm * dot(wi, wm));
+  if (walk_draw(dist, seed) <= F) return normalize(-wi + 2.0f * wm * dot(wi, wm));
   wo_out = !wi_out;
   return normalize(-eta * wi + wm * (eta * ct - ctt));
 }
@@ -818,7 +840,7 @@ PT_D float eval_dielectric_phase(uint32_t dist, const float3& wi, const float3& 
 // Conductor phase sample / eval, GGX :390-409 / Beckmann :423-442.
 PT_D float3 sample_conductor_phase(uint32_t dist, const float3& wi, float3& wm, uint32_t& seed, float ax, float ay, int* capped)
 {
-  float z1 = rnd_tea(seed), z2 = rnd_tea(seed);
+  float z1 = walk_draw(dist, seed), z2 = walk_draw(dist, seed);
   wm = sample_vndf(dist, wi, ax, ay, z1, z2, capped);
   return -wi + 2.0f * wm * dot(wi, wm);
 }
@@ -831,7 +853,7 @@ PT_D float eval_conductor_phase(uint32_t dist, const float3& wi, const float3& w
 // Diffuse phase sample / eval, GGX :342-387 / Beckmann :375-420.
 PT_D float3 sample_diffuse_phase(uint32_t dist, const float3& wi, float3& wm, uint32_t& seed, float ax, float ay, int* capped)
 {
-  float z1 = rnd_tea(seed), z2 = rnd_tea(seed), z3 = rnd_tea(seed), z4 = rnd_tea(seed);
+  float z1 = walk_draw(dist, seed), z2 = walk_draw(dist, seed), z3 = walk_draw(dist, seed), z4 = walk_draw(dist, seed);
   wm = sample_vndf(dist, wi, ax, ay, z1, z2, capped);
   float3 w1, w2;
   create_onb(wm, w1, w2);
@@ -846,7 +868,7 @@ PT_D float3 sample_diffuse_phase(uint32_t dist, const float3& wi, float3& wm, ui
 }
 PT_D float eval_diffuse_phase(uint32_t dist, const float3& wi, const float3& wo, float3& wm, float ax, float ay, uint32_t& seed, int* capped)
 {
-  float z1 = rnd_tea(seed), z2 = rnd_tea(seed);
+  float z1 = walk_draw(dist, seed), z2 = walk_draw(dist, seed);
   wm = sample_vndf(dist, wi, ax, ay, z1, z2, capped);
   if (dist == GGX) return 1.0f / kPi * fmaxf(0.0f, dot(wo, wm));
   return 1.0f * kInvPi * fmaxf(0.0f, dot(wo, wm));
@@ -860,7 +882,7 @@ PT_D float3 ms_dielectric_sample(uint32_t dist, const float3& lwi, float eta, fl
   bool out = (-wo.z) > 0;
   for (int it = 0;; ++it) {
     if (it >= kWalkCap) { *capped = 1; break; }
-    float z = rnd_tea(seed);
+    float z = walk_draw(dist, seed);
     hr = sample_height(dist, out ? wo : -wo, out ? hr : -hr, z, ax, ay);
     if (!out) hr = -hr;
     if (hr == kDefaultMax || hr == -kDefaultMax) break;
@@ -886,7 +908,7 @@ PT_D float ms_dielectric_eval(uint32_t dist, const float3& wi, const float3& wo,
     if (dist == GGX) { if (!(order == 0 || cur < (int)order)) break; }
     else { if (!(order == 0 || (uint32_t)cur <= order)) break; }
     if (it >= kWalkCap) { *capped = 1; break; }
-    float z = rnd_tea(seed);
+    float z = walk_draw(dist, seed);
     hr = sample_height(dist, wr_out ? wr : -wr, wr_out ? hr : -hr, z, ax, ay);
     if (!wr_out) hr = -hr;
     if (hr == kDefaultMax || hr == -kDefaultMax || isinf(hr)) break;
@@ -911,7 +933,7 @@ PT_D float3 ms_conductor_sample(uint32_t dist, const float3& wi, const Cx3& eta,
   weight = f3s(1.0f);
   for (int it = 0;; ++it) {
     if (it >= kWalkCap) { *capped = 1; break; }
-    float u = rnd_tea(seed);
+    float u = walk_draw(dist, seed);
     hr = sample_height(dist, wo, hr, u, ax, ay);
     if (hr == kDefaultMax) break;
     order++;
@@ -931,7 +953,7 @@ PT_D float3 ms_conductor_eval(uint32_t dist, const float3& wi, const float3& wo,
   int cur = 0;
   for (int it = 0; order == 0 || cur < (int)order; ++it) {
     if (it >= kWalkCap) { *capped = 1; break; }
-    float u = rnd_tea(seed);
+    float u = walk_draw(dist, seed);
     hr = sample_height(dist, wr, hr, u, ax, ay);
     if (hr == kDefaultMax) break;
     cur++;
@@ -955,7 +977,7 @@ PT_D float3 ms_diffuse_sample(uint32_t dist, const float3& wi, float ax, float a
   float3 wo = -wi;
   wm = f3(0.0f, 0.0f, 1.0f);
   while (order < 100u) {
-    float u = rnd_tea(seed);
+    float u = walk_draw(dist, seed);
     hr = sample_height(dist, wo, hr, u, ax, ay);
     if (hr == kDefaultMax) break;
     order++;
@@ -973,7 +995,7 @@ PT_D float3 ms_diffuse_eval(uint32_t dist, const float3& wi, const float3& wo, f
   int cur = 0;
   for (int it = 0; order == 0 || cur < (int)order; ++it) {
     if (it >= kWalkCap) { *capped = 1; break; }
-    float u = rnd_tea(seed);
+    float u = walk_draw(dist, seed);
     hr = sample_height(dist, wr, hr, u, ax, ay);
     if (hr == kDefaultMax) break;
     cur++;

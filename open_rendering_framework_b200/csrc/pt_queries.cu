@@ -7,6 +7,7 @@
 // at large n).  The FP64 variant derives the coefficients and evaluates the dipole in double.
 // pt_microfacet_queries: one random walk per thread (2-4 tea draws and an erf / erfinv per step),
 // one kernel instance per (op, distribution) so that a launch holds only the code it runs.
+#define PT_OUTLINE_TEA_BECKMANN
 #include <cmath>
 #include <cstring>
 
