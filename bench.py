@@ -82,7 +82,8 @@ UNIT = "Mpath-samples/s"
 WORKLOAD = ("single-scene render 512x512, 64 spp, max depth 8, Russian roulette from depth 3: 12-triangle diffuse box, "
             "81,920-triangle GGX conductor icosphere, 20,480-triangle Beckmann rough-dielectric icosphere, quad light")
 EXTEND_BYTES_PER_SEGMENT = 56  # queue id 4 + ray 32 + hit record 16 + material-queue append 4
-GATHER_INSTR_PER_PAIR = 256    # thread instructions per (gather, probe) pair of k_gather, from its ncu capture
+GATHER_INSTR_PER_PAIR = 303    # thread instructions per (gather, probe) pair of k_gather, from its ncu capture
+#                                (they issue to the ALU and FMA pipes together, so the bound is instruction issue)
 
 
 def parse():
@@ -941,11 +942,11 @@ def batched_roofline(st, clocks, local):
               "algorithmic_bytes_per_segment": EXTEND_BYTES_PER_SEGMENT, "traffic": None,
               "extend_share_of_pass": st.extend_ms / st.gpu_ms if st.gpu_ms else None,
               "segments_per_path": st.segments / max(1, st.path_samples)}
-    alu_peak = n_sm * 64 * sm_mhz * 1e6 / GATHER_INSTR_PER_PAIR / 1e9
+    alu_peak = n_sm * 128 * sm_mhz * 1e6 / GATHER_INSTR_PER_PAIR / 1e9
     pairs = st.dipole_pairs / gat_s / 1e9 if gat_s > 0 else None
     gather = {"bound": "alu", "kernel": "k_gather (dipole gathers: one MD5 draw per (gather, probe) pair)",
               "achieved": pairs, "peak": alu_peak, "unit": "Gpair/s", "frac": pairs / alu_peak if pairs else None,
-              "peak_source": "INT32 pipe: 64 lanes/clk/SM x SMs x median SM clock / %d thread instructions per pair "
+              "peak_source": "instruction issue: 128 lanes/clk/SM x SMs x median SM clock / %d thread instructions per pair "
                              "(ncu capture of the subsurface configuration's gather)" % GATHER_INSTR_PER_PAIR,
               "traffic": None, "gather_share_of_pass": st.gather_ms / st.gpu_ms if st.gpu_ms else None,
               "pairs_per_gather": st.dipole_pairs / max(1, st.dipole_gathers)}
@@ -1164,13 +1165,13 @@ def adjoint_roofline(fst, ast, clocks, local):
     top = max(parts, key=parts.get)
     if top.endswith("gather"):
         s = fst if top.startswith("forward") else ast
-        alu_peak = n_sm * 64 * sm_mhz * 1e6 / GATHER_INSTR_PER_PAIR / 1e9
+        alu_peak = n_sm * 128 * sm_mhz * 1e6 / GATHER_INSTR_PER_PAIR / 1e9
         achieved = s.dipole_pairs / (s.gather_ms * 1e-3) / 1e9 if s.gather_ms else None
         kernel = "k_gather (forward dipole gathers)" if top.startswith("forward") else \
             "k_gather<true> (the adjoint pass's dipole gathers: the MD5 chain replayed, derivatives of accepted pairs)"
         out = {"bound": "alu", "kernel": kernel, "achieved": achieved, "peak": alu_peak, "unit": "Gpair/s",
                "frac": achieved / alu_peak if achieved else None,
-               "peak_source": "INT32 pipe: 64 lanes/clk/SM x SMs x median SM clock / %d thread instructions per pair of the "
+               "peak_source": "instruction issue: 128 lanes/clk/SM x SMs x median SM clock / %d thread instructions per pair of the "
                               "forward gather (ncu)%s" % (GATHER_INSTR_PER_PAIR, "" if top.startswith("forward") else
                                                           "; the adjoint gather does more per pair, so frac is a lower bound"),
                "traffic": None, "pairs_per_gather": s.dipole_pairs / max(1, s.dipole_gathers)}
@@ -1492,14 +1493,14 @@ def run_ours(args, world, rank, local):
                 "giga_rays_per_s": (st.segments + st.shadow_rays) / (st.gpu_ms * 1e-3) / 1e9,
                 "record": "profiles/k_extend_single_scene_ncu.csv" if rec else None}
     if args.workload == "subsurface":
-        # integer-issue bound: 64 INT32 lanes per clock per SM at the sampled SM clock, divided by the
-        # thread instructions one pair takes (ncu capture of k_gather)
+        # issue bound: 128 lanes per clock per SM at the sampled SM clock, divided by the thread
+        # instructions one pair takes (ncu capture of k_gather)
         sm_mhz = clocks.summary().get("sm_mhz") or 1965.0
-        alu_peak = torch.cuda.get_device_properties(local).multi_processor_count * 64 * sm_mhz * 1e6 / GATHER_INSTR_PER_PAIR / 1e9
+        alu_peak = torch.cuda.get_device_properties(local).multi_processor_count * 128 * sm_mhz * 1e6 / GATHER_INSTR_PER_PAIR / 1e9
         achieved_g = st.dipole_pairs / (st.gather_ms * 1e-3) / 1e9 if st.gather_ms else None
         roofline = {"bound": "alu", "kernel": "k_gather (dipole gathers: one MD5 draw per (gather, probe) pair)",
                     "achieved": achieved_g, "unit": "Gpair/s", "peak": alu_peak,
-                    "peak_source": "INT32 pipe: 64 lanes/clk/SM x SMs x median SM clock / %d thread instructions per pair (ncu)" %
+                    "peak_source": "instruction issue: 128 lanes/clk/SM x SMs x median SM clock / %d thread instructions per pair (ncu)" %
                                    GATHER_INSTR_PER_PAIR,
                     "frac": achieved_g / alu_peak if achieved_g else None, "traffic": None,
                     "gather_share_of_render": st.gather_ms / st.gpu_ms if st.gpu_ms else None,
