@@ -1222,7 +1222,15 @@ template <class K> inline int full_wave(K kernel)
 //   with translucent objects (more launches a pass): 1 M 2370 / 1701, 2 M 3550 / 2861; adjoint 3.1 M 20394 / 20381
 //   batch of ten scenes (the wavefront's multi-scene traversal spills): 1.9 M 3296 / 2453, 7.5 M 7177 / 6909,
 //   30 M in chunks of 16 M 23177 / 23526
-inline uint64_t pool_max_paths(bool translucent, bool multi) { return translucent ? (multi ? 1ull << 23 : 1ull << 21) : (multi ? 1ull << 21 : 1ull << 20); }
+// With several contexts rendering at once the others fill the wavefront's gaps and the lines lie lower, so they
+// are drawn there.  Three contexts in turn (wavefront / pools): sky 0.78 M paths 758 / 716, 1.04 M 854 / 906;
+// single scene 0.79 M 1631 / 1545; all programs 0.59 M 1322 / 1208, 0.79 M 1670 / 1788 and 2017 / 2312;
+// translucent 1.3 M 2034 / 1608.
+inline uint64_t pool_max_paths(bool translucent, bool all_programs, bool multi)
+{
+  const uint64_t single = translucent ? 3ull << 19 : all_programs ? 1ull << 19 : 3ull << 18;
+  return multi ? (translucent ? 1ull << 23 : 2 * single) : single;
+}
 enum PoolPrograms { POOL_BASIC = 0, POOL_TRANSLUCENT = 1 /* and smooth translucent objects */, POOL_ALL = 2 };
 pt_status launch_path_pools(const SceneDev& S0, const WfDev& w, uint64_t n, bool multi, bool adjoint, PoolPrograms programs, int refill,
                             cudaStream_t stream);
