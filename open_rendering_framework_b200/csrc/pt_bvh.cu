@@ -277,7 +277,7 @@ bool build_bvh(const float* tri_pos, uint32_t n_tris, BvhHost& out, const BvhPar
   return out.depth < 64;
 }
 
-float scene_diagonal(const float* tri_pos, uint32_t n)
+float scene_diagonal(const float* tri_pos, uint32_t n, float* reach)
 {
   float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
   for (size_t i = 0; i < (size_t)n * 3; ++i)
@@ -287,6 +287,10 @@ float scene_diagonal(const float* tri_pos, uint32_t n)
     }
   double d2 = 0.0;
   for (int k = 0; k < 3; ++k) d2 += (double)(hi[k] - lo[k]) * (hi[k] - lo[k]);
+  if (reach) {
+    *reach = 0.0f;
+    for (int k = 0; k < 3 && n; ++k) *reach = std::max(*reach, std::max(std::fabs(lo[k]), std::fabs(hi[k])));
+  }
   return n ? (float)std::sqrt(d2) : 0.0f;
 }
 

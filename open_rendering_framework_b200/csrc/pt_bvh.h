@@ -40,6 +40,6 @@ bool build_bvh4(const BvhHost& bvh2, std::vector<float4>& nodes4, int& depth4, c
 
 // The diagonal of the bounding box of n triangles (9 floats each): the scale of the box tests' margin
 // (SceneDev::trav_scale).
-float scene_diagonal(const float* tri_pos, uint32_t n);
+float scene_diagonal(const float* tri_pos, uint32_t n, float* reach = nullptr);
 
 }  // namespace pt

@@ -19,6 +19,7 @@ SceneDev Context::view() const
   s.nodes = d_nodes.as<float4>();
   s.nodes4 = has_bvh4 && use_bvh4 ? d_nodes4.as<float4>() : nullptr;
   s.trav_scale = trav_scale;
+  s.trav_reach = trav_reach;
   s.tri_v0 = d_v0.as<float4>();
   s.tri_e1 = d_e1.as<float4>();
   s.tri_e2 = d_e2.as<float4>();
@@ -340,7 +341,7 @@ __global__ void __launch_bounds__(kQueryBlock, 1024 / kQueryBlock) k_trace_wide(
         h.t = tmax;
         h.u = h.v = 0.0f;
         h.prim = -1;
-        if (wide_ray(o, d, tmin, g.trav_scale)) {
+        if (wide_ray(o, d, tmin, g)) {
           rp = ray_pre4(o, d, g.trav_scale);
           stack4_init(s4, stk + threadIdx.x, kQueryBlock, spill4);
           cur = 0;
@@ -796,7 +797,7 @@ pt_status pt_build(pt_ctx* ctx)
   Context& c = ctx->c;
   if (c.n_tris == 0) return fail(PT_NOT_READY, "pt_build: no meshes");
   PT_CHECK_CUDA(cudaSetDevice(c.device), "cudaSetDevice");
-  c.trav_scale = scene_diagonal(c.tri_pos.data(), c.n_tris);
+  c.trav_scale = scene_diagonal(c.tri_pos.data(), c.n_tris, &c.trav_reach);
   const auto t0 = std::chrono::steady_clock::now();
   pt_status st = PT_OK;
   bool on_device = false;

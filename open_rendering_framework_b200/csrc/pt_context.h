@@ -216,6 +216,7 @@ struct Context {
   bool use_bvh4 = true;  // option "bvh4": the persistent traversal kernels walk the 4-wide BVH
   int bvh_builder = 0;   // option "bvh_builder": 0 host binned SAH, 1 device LBVH
   float trav_scale = 0.0f;  // diagonal of the triangles' bounding box (the box tests' margin), set by pt_build
+  float trav_reach = 0.0f;  // largest coordinate magnitude of the triangles (wide_ray), set by pt_build
   pt_build_info build_info{};
   DevBuf d_build_scratch;  // the device builder's temporaries, kept for rebuilds
   DevBuf d_scat, d_trans_objs, d_trans_pos;

@@ -149,7 +149,7 @@ __device__ __forceinline__ float3 shading_normal(const SceneDev& S, const int4& 
 static __device__ __noinline__ bool occluded(const SceneDev& S, float3 o, float3 d, float tmin, float tmax)
 {
   const TravGeom g = trav_geom(S);
-  const bool hit = g.nodes4 && wide_ray(o, d, tmin, g.trav_scale) ? trace_any_wide(g, o, d, tmin, tmax) : trace_any(g, o, d, tmin, tmax);
+  const bool hit = g.nodes4 && wide_ray(o, d, tmin, g) ? trace_any_wide(g, o, d, tmin, tmax) : trace_any(g, o, d, tmin, tmax);
   return hit || (S.n_ana && ana_any(S, o, d, tmin, tmax));
 }
 
