@@ -1437,7 +1437,7 @@ pt_status pass_resources(Context& E, const PassLayout& L, const std::vector<Scen
   if (st == PT_OK && L.dual) st = ensure_wavefront(E.wf2, L.cap_paths);
   // a small pass's probe paths run beside its camera paths, in a wavefront of their own where memory allows
   E.probes_beside = st == PT_OK && L.sss && E.opt.pool && E.opt.overlap && L.cap_probes > 0 && L.cap_probes <= kProbesBesideMax &&
-                    (E.opt.pool == 2 || L.cap_paths <= pool_max_paths(true, false, scenes.size() > 1)) && ensure_wavefront(E.wf2, L.cap_probes) == PT_OK;
+                    (E.opt.pool == 2 || L.cap_paths <= pool_max_paths(true, L.ms || L.layered || L.rough, scenes.size() > 1)) && ensure_wavefront(E.wf2, L.cap_probes) == PT_OK;
   if (st == PT_OK && L.sss) st = ensure_sss(E, E.wf.cap, L.g_slots, L.cap_probes, L.cap_sets);
   if (st == PT_OK) st = E.d_scene_tab.reserve(scenes.size() * sizeof(SceneDev), "scene table");
   if (st == PT_OK) st = E.d_item_tab.reserve(std::max<size_t>(L.items.size(), 1) * sizeof(ItemDev), "item table");

@@ -1216,20 +1216,25 @@ template <class K> inline int full_wave(K kernel)
 // Up to how many paths a chunk runs through pools instead of the wavefront's launches.  A bounce of the
 // wavefront costs eleven launches and waits for its slowest ray on the whole GPU, which a small chunk
 // cannot hide; a pool's warps wait for their block's slowest ray instead, and its one kernel holds every
-// program, which a large chunk pays for.  Measured (wavefront / pools, us a render):
-//   single scene (subdiv 5, depth 8): 16 K paths 1181 / 494, 262 K 1530 / 940, 1 M 2795 / 2464, 2 M 4300 / 4473
-//   layered, multiple scattering: 262 K 5161 / 3861, 1 M 10834 / 10328; analytic lights: 1 M 2761 / 2652
-//   with translucent objects (more launches a pass): 1 M 2370 / 1701, 2 M 3550 / 2861; adjoint 3.1 M 20394 / 20381
-//   batch of ten scenes (the wavefront's multi-scene traversal spills): 1.9 M 3296 / 2453, 7.5 M 7177 / 6909,
-//   30 M in chunks of 16 M 23177 / 23526
-// With several contexts rendering at once the others fill the wavefront's gaps and the lines lie lower, so they
-// are drawn there.  Three contexts in turn (wavefront / pools): sky 0.78 M paths 758 / 716, 1.04 M 854 / 906;
-// single scene 0.79 M 1631 / 1545; all programs 0.59 M 1322 / 1208, 0.79 M 1670 / 1788 and 2017 / 2312;
-// translucent 1.3 M 2034 / 1608.
+// program, which a large chunk pays for.  The other contexts' work fills the wavefront's gaps where several
+// render at once, so the lines lie lower there, and that is where those of one scene are drawn: a program
+// that renders in one context alone could go on to about twice the paths.  Measured (wavefront / pools, us a
+// render; three contexts in turn, then one alone):
+//   basic (subdiv 5, depth 8)   0.79 M paths 1888 / 1673, 2182 / 1816; 1.57 M 3023 / 3111, 3445 / 3247
+//   layered, multiple scattering   0.52 M 2680 / 2656, 3769 / 2780; 1.05 M 3923 / 4011, 4998 / 4276
+//   smooth translucent   1.57 M 3894 / 3263, 4713 / 3619; 2.1 M 4810 / 4236, 5583 / 4584
+//   translucent and all programs   1.57 M 4423 / 4055, 5496 / 4431 (rough, Walter), 5509 / 5220, 6728 / 5718 (rough,
+//   multiple scattering), 7922 / 7015, 10004 / 7563 (beside layered); 2.1 M 5414 / 5250, 6782 / 6771, 9813 / 9082
+// Passes of several scenes (the wavefront's multi-scene traversal spills; four scenes in one batch):
+//   basic   1.05 M 2881 / 2600, 2.1 M 4638 / 4805; layered   1.05 M 5225 / 4605, 4.2 M 14576 / 14887
+//   smooth translucent   4.2 M 9672 / 9137, 8.4 M 17746 / 17688, 12.6 M 25939 / 26366
+//   translucent and all programs   2.1 M 8276 / 7693 (one scene of each kind), 7977 / 7487 (rough), 11685 / 10055 (beside
+//   layered); 4.2 M 12670 / 14277, 13586 / 13889, 19860 / 18731; 8.4 M 21870 / 27563
 inline uint64_t pool_max_paths(bool translucent, bool all_programs, bool multi)
 {
+  if (multi && translucent) return all_programs ? 1ull << 21 : 1ull << 23;
   const uint64_t single = translucent ? 3ull << 19 : all_programs ? 1ull << 19 : 3ull << 18;
-  return multi ? (translucent ? 1ull << 23 : 2 * single) : single;
+  return multi ? 2 * single : single;
 }
 enum PoolPrograms { POOL_BASIC = 0, POOL_TRANSLUCENT = 1 /* and smooth translucent objects */, POOL_ALL = 2 };
 pt_status launch_path_pools(const SceneDev& S0, const WfDev& w, uint64_t n, bool multi, bool adjoint, PoolPrograms programs, int refill,
