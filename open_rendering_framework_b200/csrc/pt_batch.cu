@@ -70,6 +70,8 @@ std::vector<uint64_t> graph_key(const Context& E, const PassLayout& L, const std
     k.push_back((uint64_t)(uintptr_t)p);
   k.push_back(E.wf.cap);
   k.push_back(E.wf2.cap);
+  k.push_back((uint64_t)(uintptr_t)E.probe_wf.buf.p);
+  k.push_back(E.probe_wf.cap);
   k.push_back(E.probes_beside ? 1 : 0);
   k.push_back((uint64_t)E.opt.extend_mode);
   k.push_back((uint64_t)E.opt.refill);

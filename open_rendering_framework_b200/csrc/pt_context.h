@@ -90,6 +90,16 @@ struct Wavefront {
   DevBuf pc_pos, pc_wl, pc_nrm, pc_tr, pc_cnt;// probes with L != 0, compacted in order per (frame, object)
 };
 
+// What path pools read of a wavefront, for the probe paths that run beside the camera paths: one
+// allocation for `cap` paths, the counters first (a first render in a new context pays for every
+// allocation; the wavefront's own fifteen made it slower than the pools gained).
+struct ProbeWavefront {
+  uint64_t cap = 0;
+  DevBuf buf;
+};
+constexpr size_t kProbeCounterBytes = 256;
+constexpr size_t kProbePathBytes = 7 * 16 + 2 * 16 + 4 + 2;  // seven float4, two records of a pair, queue entry, item
+
 // Counter slots in Wavefront::counters.
 enum CounterSlot {
   CNT_ACTIVE_A = 0,
@@ -258,8 +268,9 @@ struct Context {
   cudaStream_t stream2 = nullptr, side2[2] = {nullptr, nullptr};
   cudaEvent_t ev2_fork = nullptr, ev2_join = nullptr, ev2_shade = nullptr, ev2_shadow = nullptr;
   cudaEvent_t ev_start = nullptr, ev_acc = nullptr, ev_end2 = nullptr;
-  bool pass_dual = false;  // the last pass ran two pipelines, or probes beside paths (its counters are in wf and wf2)
-  bool probes_beside = false;  // the current pass may run its probe paths in wf2, beside the camera paths
+  ProbeWavefront probe_wf;     // the probe paths beside the camera paths (on stream2, between ev_start and ev_end2)
+  const DevBuf* pass_second = nullptr;  // beside wf's, the counters of the last pass: wf2's (two pipelines), the probe wavefront's, or none
+  bool probes_beside = false;  // the current pass may run its probe paths in probe_wf, beside the camera paths
   bool profile = false;
   std::vector<cudaEvent_t> prof_events;  // pairs around each extend and gather launch when profiling
   std::vector<int> prof_kind;            // PROF_EXTEND or PROF_GATHER per pair

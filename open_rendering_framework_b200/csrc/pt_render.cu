@@ -1209,8 +1209,44 @@ __global__ void k_geo_normals(SceneDev S, float4* geo)
   }
 }
 
-// Probe paths of a chunk that may run beside its camera paths: 47 MB of wavefront at most.
+// Probe paths of a chunk that may run beside its camera paths: 39 MB of wavefront at most.
 constexpr uint64_t kProbesBesideMax = 1ull << 18;
+static_assert(kCounters * 4 <= kProbeCounterBytes, "the probe wavefront's counters");
+static pt_status ensure_probe_wavefront(ProbeWavefront& p, uint64_t cap)
+{
+  if (p.cap >= cap && p.buf.p) return PT_OK;
+  p.cap = 0;
+  const uint64_t n = (cap + 7) / 8 * 8;  // every array starts on a 16-byte boundary
+  pt_status st = p.buf.reserve(kProbeCounterBytes + n * kProbePathBytes, "probe wavefront");
+  if (st == PT_OK) p.cap = n;
+  return st;
+}
+// Its device view: the arrays that the pools and the probe kernels read; the others stay as they are in v.
+static void probe_view(const ProbeWavefront& p, WfDev& v)
+{
+  char* at = p.buf.as<char>();
+  auto take = [&](size_t bytes) {
+    char* r = at;
+    at += bytes;
+    return r;
+  };
+  v.cap = p.cap;
+  v.cnt = reinterpret_cast<uint32_t*>(take(kProbeCounterBytes));
+  float4* rays = reinterpret_cast<float4*>(take(p.cap * 32));
+  float4* state = reinterpret_cast<float4*>(take(p.cap * 32));
+  v.ray_o = Field2<float4>{rays};
+  v.ray_d = Field2<float4>{rays + 1};
+  v.thr = Field2<float4>{state};
+  v.rng = Field2<uint4>{reinterpret_cast<uint4*>(state + 1)};
+  for (float4** f : {&v.rad, &v.hit, &v.sh_o, &v.sh_d, &v.sh_c}) *f = reinterpret_cast<float4*>(take(p.cap * 16));
+  v.q_in = reinterpret_cast<uint32_t*>(take(p.cap * 4));
+  v.path_item = reinterpret_cast<uint16_t*>(take(p.cap * 2));
+  v.q_out = v.q_mat = v.bin = v.sh_pid = nullptr;
+  v.cls_of = nullptr;
+  v.g_a = v.g_b = v.g_d = v.adj_a = v.adj_b = nullptr;
+  v.g_c = nullptr;
+  v.g_slots = 0;
+}
 
 static pt_status ensure_wavefront(Wavefront& wf, uint64_t cap)
 {
@@ -1437,7 +1473,7 @@ pt_status pass_resources(Context& E, const PassLayout& L, const std::vector<Scen
   if (st == PT_OK && L.dual) st = ensure_wavefront(E.wf2, L.cap_paths);
   // a small pass's probe paths run beside its camera paths, in a wavefront of their own where memory allows
   E.probes_beside = st == PT_OK && L.sss && E.opt.pool && E.opt.overlap && L.cap_probes > 0 && L.cap_probes <= kProbesBesideMax &&
-                    (E.opt.pool == 2 || L.cap_paths <= pool_max_paths(true, L.ms || L.layered || L.rough, scenes.size() > 1)) && ensure_wavefront(E.wf2, L.cap_probes) == PT_OK;
+                    (E.opt.pool == 2 || L.cap_paths <= pool_max_paths(true, L.ms || L.layered || L.rough, scenes.size() > 1)) && ensure_probe_wavefront(E.probe_wf, L.cap_probes) == PT_OK;
   if (st == PT_OK && L.sss) st = ensure_sss(E, E.wf.cap, L.g_slots, L.cap_probes, L.cap_sets);
   if (st == PT_OK) st = E.d_scene_tab.reserve(scenes.size() * sizeof(SceneDev), "scene table");
   if (st == PT_OK) st = E.d_item_tab.reserve(std::max<size_t>(L.items.size(), 1) * sizeof(ItemDev), "item table");
@@ -1450,9 +1486,14 @@ pt_status pass_resources(Context& E, const PassLayout& L, const std::vector<Scen
   for (cudaEvent_t* ev : {&E.ev_fork, &E.ev_join, &E.ev_shade, &E.ev_shadow})
     if (!*ev) PT_CHECK_CUDA(cudaEventCreateWithFlags(ev, cudaEventDisableTiming), "stream event");
   if (L.dual || E.probes_beside) {
-    for (cudaStream_t* sd : {&E.stream2, &E.side2[0], &E.side2[1]})
+    if (!E.stream2) PT_CHECK_CUDA(cudaStreamCreateWithFlags(&E.stream2, cudaStreamNonBlocking), "second pipeline stream");
+    for (cudaEvent_t* ev : {&E.ev_start, &E.ev_end2})
+      if (!*ev) PT_CHECK_CUDA(cudaEventCreateWithFlags(ev, cudaEventDisableTiming), "stream event");
+  }
+  if (L.dual) {
+    for (cudaStream_t* sd : {&E.side2[0], &E.side2[1]})
       if (!*sd) PT_CHECK_CUDA(cudaStreamCreateWithFlags(sd, cudaStreamNonBlocking), "second pipeline stream");
-    for (cudaEvent_t* ev : {&E.ev2_fork, &E.ev2_join, &E.ev2_shade, &E.ev2_shadow, &E.ev_start, &E.ev_acc, &E.ev_end2})
+    for (cudaEvent_t* ev : {&E.ev2_fork, &E.ev2_join, &E.ev2_shade, &E.ev2_shadow, &E.ev_acc})
       if (!*ev) PT_CHECK_CUDA(cudaEventCreateWithFlags(ev, cudaEventDisableTiming), "stream event");
   }
   PT_CHECK_CUDA(cudaMemcpyAsync(E.d_scene_tab.p, scenes.data(), scenes.size() * sizeof(SceneDev), cudaMemcpyHostToDevice, E.stream), "scene table");
@@ -1513,7 +1554,7 @@ pt_status launch_pass(Context& E, const PassLayout& L, const std::vector<SceneDe
   Wavefront* const wf_of[2] = {&c.wf, dual ? &c.wf2 : &c.wf};
   WfDev w = w_of[0];
   Wavefront* wf = wf_of[0];
-  c.pass_dual = dual || c.probes_beside;
+  c.pass_second = dual ? &c.wf2.counters : c.probes_beside ? &c.probe_wf.buf : nullptr;
   Wavefront& wf0 = c.wf;
   SssDev g;
   memset(&g, 0, sizeof(g));
@@ -1553,7 +1594,7 @@ pt_status launch_pass(Context& E, const PassLayout& L, const std::vector<SceneDe
     PT_CHECK_CUDA(cudaStreamWaitEvent(c.stream2, c.ev_start, 0), "second pipeline start");
     PT_CHECK_CUDA(cudaMemsetAsync(w_of[1].cnt, 0, kCounters * 4, c.stream2), "reset counters");
   }
-  if (c.probes_beside) PT_CHECK_CUDA(cudaMemsetAsync(c.wf2.counters.p, 0, kCounters * 4, c.stream), "reset counters");
+  if (c.probes_beside) PT_CHECK_CUDA(cudaMemsetAsync(c.probe_wf.buf.p, 0, kCounters * 4, c.stream), "reset counters");
   c.prof_pairs = 0;
   pt_status st = PT_OK;
   // CUDA events around the launches whose device time the stats report (when profiling is on)
@@ -1727,16 +1768,10 @@ pt_status launch_pass(Context& E, const PassLayout& L, const std::vector<SceneDe
     const uint64_t n_paths = L.chunk_paths[k], n_probes = L.chunk_probes[k];
     // the camera paths do not read the probes (their gathers are evaluated at the end), so where both are
     // small the probe pass runs on a stream and in a wavefront of its own until the gathers
-    const bool beside = n_probes && c.probes_beside && n_probes <= c.wf2.cap && by_pools(n_paths) && by_pools(n_probes);
+    const bool beside = n_probes && c.probes_beside && n_probes <= c.probe_wf.cap && by_pools(n_paths) && by_pools(n_probes);
     if (beside) {
-      WfDev p = make_w(c.wf2);
-      p.items = w.items;
-      p.n_items = w.n_items;
-      p.multi = w.multi;
-      p.scene0 = w.scene0;
-      p.adj_a = p.adj_b = nullptr;
-      p.q_in = c.wf2.q_a.as<uint32_t>();
-      p.q_out = c.wf2.q_b.as<uint32_t>();
+      WfDev p = w;
+      probe_view(c.probe_wf, p);
       p.in_slot = CNT_ACTIVE_A;
       p.out_slot = CNT_ACTIVE_B;
       PT_CHECK_CUDA(cudaEventRecord(c.ev_start, s_main), "probe pass start");
@@ -1903,8 +1938,8 @@ pt_status pt_get_render_stats(pt_ctx* ctx, pt_render_stats* out)
   if (c.stats_pending && c.wf.counters.p) {
     uint32_t h[kCounters], h2[kCounters];
     PT_CHECK_CUDA(cudaMemcpy(h, c.wf.counters.p, sizeof(h), cudaMemcpyDeviceToHost), "read counters");
-    const bool two = c.pass_dual && c.wf2.counters.p;  // a dual pass counts in both wavefronts
-    if (two) PT_CHECK_CUDA(cudaMemcpy(h2, c.wf2.counters.p, sizeof(h2), cudaMemcpyDeviceToHost), "read counters");
+    const bool two = c.pass_second && c.pass_second->p;
+    if (two) PT_CHECK_CUDA(cudaMemcpy(h2, c.pass_second->p, sizeof(h2), cudaMemcpyDeviceToHost), "read counters");
     auto rd64 = [&](int slot) {
       unsigned long long v, v2 = 0;
       memcpy(&v, h + slot, 8);

@@ -1,0 +1,24 @@
+"""The probe paths that run beside the camera paths: what their wavefront holds, and when it is used."""
+import pytest
+
+from open_rendering_framework_b200 import scene as sc
+from open_rendering_framework_b200 import scenes
+
+pytestmark = pytest.mark.gpu
+
+
+def test_probe_wavefront_holds_only_what_pools_read():
+    """A first render with the probe pass on its own wavefront (option overlap 1) takes at most the 150 bytes a
+    probe path that the pools read, and 4 MB of granularity, more than one without (overlap 0)."""
+    torch = pytest.importorskip("torch")
+    probes = 200_000
+    used = []
+    for overlap in (0, 0, 1):  # the first round brings in the kernels' own memory
+        R = sc.Renderer(scenes.translucent_box_scene(16, 16, probe_samples=probes))
+        R.set_option("overlap", overlap)
+        before = torch.cuda.mem_get_info()[0]
+        R.render(1)
+        R.sync()
+        used.append(before - torch.cuda.mem_get_info()[0])
+        R.close()
+    assert 100 * probes < used[2] - used[1] <= 150 * probes + (4 << 20), used
