@@ -26,6 +26,7 @@ struct pt_batch {
   cudaGraphExec_t exec = nullptr;
   std::vector<uint64_t> key;     // what the captured graph depends on
   uint64_t graph_kernels = 0;    // kernel nodes of the captured graph
+  const DevBuf* graph_second = nullptr;  // where the captured pass counts beside the wavefront (Context::pass_second)
   cudaEvent_t done = nullptr;
 };
 
@@ -157,8 +158,10 @@ pt_status render(pt_batch* b, bool graph, const std::vector<uint32_t>* frames_ov
       }
       b->key = key;
       b->graph_kernels = captured;
+      b->graph_second = E.pass_second;
       launches0 += captured;  // captured, not launched
     }
+    E.pass_second = b->graph_second;  // other passes may have run on the engine since the capture
     PT_CHECK_CUDA(cudaEventRecord(E.ev0, E.stream), "event");
     PT_CHECK_CUDA(cudaGraphLaunch(b->exec, E.stream), "graph launch");
     PT_CHECK_CUDA(cudaEventRecord(E.ev1, E.stream), "event");
