@@ -1471,8 +1471,10 @@ pt_status pass_resources(Context& E, const PassLayout& L, const std::vector<Scen
 {
   pt_status st = ensure_wavefront(E.wf, L.cap_paths);
   if (st == PT_OK && L.dual) st = ensure_wavefront(E.wf2, L.cap_paths);
-  // a small pass's probe paths run beside its camera paths, in a wavefront of their own where memory allows
+  // a small pass's probe paths run beside its camera paths, in a wavefront of their own where memory and the
+  // caller's bound on the paths in flight allow
   E.probes_beside = st == PT_OK && L.sss && E.opt.pool && E.opt.overlap && L.cap_probes > 0 && L.cap_probes <= kProbesBesideMax &&
+                    L.cap_paths + L.cap_probes <= E.max_paths &&
                     (E.opt.pool == 2 || L.cap_paths <= pool_max_paths(true, L.ms || L.layered || L.rough, scenes.size() > 1)) && ensure_probe_wavefront(E.probe_wf, L.cap_probes) == PT_OK;
   if (st == PT_OK && L.sss) st = ensure_sss(E, E.wf.cap, L.g_slots, L.cap_probes, L.cap_sets);
   if (st == PT_OK) st = E.d_scene_tab.reserve(scenes.size() * sizeof(SceneDev), "scene table");
