@@ -280,18 +280,20 @@ template <class T> static pt_status upload(DevBuf& buf, const std::vector<T>& v,
 // ------------------------------------------------------------------ query kernels
 __global__ void k_trace_closest(SceneDev S, const float4* ot, const float4* dt, uint32_t n, int32_t* prim, float* tout, float* bary)
 {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  for (uint64_t at = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; at < n; at += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t i = (uint32_t)at;
     float4 a = ot[i], b = dt[i];
     Hit h = scene_closest(S, f3(a.x, a.y, a.z), f3(b.x, b.y, b.z), a.w, b.w);
     prim[i] = h.prim;
     tout[i] = h.prim >= 0 ? h.t : -1.0f;
-    bary[2 * i] = h.u;
-    bary[2 * i + 1] = h.v;
+    bary[bary_at(i)] = h.u;
+    bary[bary_at(i) + 1] = h.v;
   }
 }
 __global__ void k_trace_any(SceneDev S, const float4* ot, const float4* dt, uint32_t n, int32_t* hit)
 {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  for (uint64_t at = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; at < n; at += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t i = (uint32_t)at;
     float4 a = ot[i], b = dt[i];
     hit[i] = scene_any(S, f3(a.x, a.y, a.z), f3(b.x, b.y, b.z), a.w, b.w) ? 1 : 0;
   }
@@ -387,8 +389,8 @@ __global__ void __launch_bounds__(kQueryBlock, 1024 / kQueryBlock) k_trace_wide(
         if (S.n_ana) ana_closest(S, o, d, tmin, h);
         out[i] = h.prim;
         tout[i] = h.prim >= 0 ? h.t : -1.0f;
-        bary[2 * i] = h.u;
-        bary[2 * i + 1] = h.v;
+        bary[bary_at(i)] = h.u;
+        bary[bary_at(i) + 1] = h.v;
       }
       has = false;
     }
@@ -399,7 +401,7 @@ static void launch_trace_wide(const Context& c, const SceneDev& S, const float* 
 {
   // one resident wave of warps, each with an equal run of rays, at least 32
   const uint32_t warps = (uint32_t)sm_count() * 32u;
-  const uint32_t per = std::max(32u, (n + warps - 1) / warps);
+  const uint32_t per = rays_per_warp(n, warps);
   const uint32_t blocks = (uint32_t)(((uint64_t)n + (uint64_t)per * (kQueryBlock / 32) - 1) / ((uint64_t)per * (kQueryBlock / 32)));
   k_trace_wide<kAny><<<blocks, kQueryBlock, 0, c.stream>>>(S, (const float4*)o, (const float4*)d, n, per, out, t, bary);
 }

@@ -215,6 +215,14 @@ struct Hit {
   float t, u, v;
   int prim;  // original triangle index, -1 = miss
 };
+// Where the barycentrics of query ray i lie (2 floats per ray), and how many of n rays each of `warps` warps
+// takes, at least 32: in 64 bits, since n may be any uint32.
+PT_HD size_t bary_at(uint32_t i) { return 2 * (size_t)i; }
+PT_HD uint32_t rays_per_warp(uint32_t n, uint32_t warps)
+{
+  const uint32_t per = (uint32_t)(((uint64_t)n + warps - 1) / warps);
+  return per < 32u ? 32u : per;
+}
 
 // ------------------------------------------------------------------ intersection primitives
 // The box tests only prune: the triangle test alone decides hits, so a box must never be culled when

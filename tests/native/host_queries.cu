@@ -32,6 +32,8 @@ extern "C" __attribute__((visibility("default"))) void* hq_build(const float* tr
   h->S.trav_scale = scene_diagonal(tri_pos, n, &h->S.trav_reach);
   return h;
 }
+extern "C" __attribute__((visibility("default"))) unsigned long long hq_bary_at(unsigned i) { return bary_at(i); }
+extern "C" __attribute__((visibility("default"))) unsigned hq_rays_per_warp(unsigned n, unsigned warps) { return rays_per_warp(n, warps); }
 extern "C" __attribute__((visibility("default"))) void hq_free(void* h) { delete (QueryScene*)h; }
 // rays: n x 8 floats (origin, tmin, direction, tmax).  wide: whether the ray is traced over the wide BVH;
 // prim / t / any and prim2 / t2 / any2: the results over the wide BVH (where wide) and over the BVH2.

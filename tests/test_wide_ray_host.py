@@ -30,6 +30,10 @@ def lib():
     L.hq_build.restype = ctypes.c_void_p
     L.hq_build.argtypes = [ctypes.c_void_p, ctypes.c_uint]
     L.hq_free.argtypes = [ctypes.c_void_p]
+    L.hq_bary_at.restype = ctypes.c_ulonglong
+    L.hq_bary_at.argtypes = [ctypes.c_uint]
+    L.hq_rays_per_warp.restype = ctypes.c_uint
+    L.hq_rays_per_warp.argtypes = [ctypes.c_uint, ctypes.c_uint]
     L.hq_trace.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_long] + [ctypes.c_void_p] * 7
     return L
 
@@ -120,3 +124,12 @@ def test_every_unit_direction_near_an_ordinary_scene_is_admitted(lib):
     d /= np.linalg.norm(d, axis=1, keepdims=True)
     rays = np.concatenate([rng.uniform(-100, 100, (n, 3)), np.full((n, 1), 1e-4), d, np.full((n, 1), 1e27)], 1).astype(np.float32)
     assert trace(lib, tp, np.ascontiguousarray(rays))[0].all()
+
+
+@pytest.mark.parametrize("i", [0, 1, 2 ** 31 - 1, 2 ** 31, 2 ** 32 - 1])
+def test_query_indexes_hold_for_every_ray_count(lib, i):
+    """Ray i's barycentrics lie at 2 i and the warps' runs cover all of n = i rays, past 2^31 too."""
+    assert lib.hq_bary_at(i) == 2 * i
+    for warps in (32, 4736):
+        per = lib.hq_rays_per_warp(i, warps)
+        assert per == max(32, -(-i // warps)) and per * warps >= i
