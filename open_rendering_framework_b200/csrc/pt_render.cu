@@ -1784,6 +1784,7 @@ pt_status launch_pass(Context& E, const PassLayout& L, const std::vector<SceneDe
       k_probe_finish<<<grid_for(n_probes, kBlock, 16), kBlock, 0, c.stream2>>>(p, g, 0, n_probes);
       k_probe_compact<<<L.chunk_sets[k], 256, 0, c.stream2>>>(p, g);
       count_launch(4);
+      ++c.stats.extend_launches;
       PT_CHECK_CUDA(cudaEventRecord(c.ev_end2, c.stream2), "probe pass join");
     } else if (n_probes) {
       for (uint64_t j0 = 0; j0 < n_probes; j0 += w.cap) {

@@ -38,3 +38,15 @@ def test_probe_paths_keep_to_the_bound_on_paths_in_flight(max_paths, beside):
         R.close()
     in_order = 3 * -(-6000 // (40 * 31)) + 1 + 5  # generate, trace, finish per 1,240 probes; compact; the camera paths
     assert launches == [9 if beside else in_order, in_order], launches
+
+
+def test_launches_that_trace_paths_are_counted_beside_and_in_order():
+    """extend_launches counts a pool launch for the probe paths and one for the camera paths, on either stream."""
+    got = []
+    for overlap in (1, 0):
+        R = sc.Renderer(scenes.translucent_box_scene(40, 31, probe_samples=200))
+        R.set_option("overlap", overlap)
+        R.render(2)
+        got.append(R.stats().extend_launches)
+        R.close()
+    assert got == [2, 2]
