@@ -469,7 +469,8 @@ pt_status pt_batch_get_stats(pt_batch* batch, pt_render_stats* out);
 /* Times short renders (min(frames_per_render, frames_per_trial) frames of every scene) over the
  * engine options -- extend kernel, warp refill threshold, paths per wavefront chunk (the queue tile),
  * then the material binning's positions per thread (the sort granularity) for the winner -- and keeps
- * the fastest.  The trials render from frame 0, so every scene's accumulation restarts at frame 0. */
+ * the fastest.  The trials take the schedule of the full render (bounce by bounce or path pools, which
+ * do not bin, so that search is left out for them).  They render from frame 0, so every scene's accumulation restarts at frame 0. */
 pt_status pt_batch_autotune(pt_batch* batch, uint32_t frames_per_trial, pt_tune_result* out);
 
 /* ---------------------------------------------------------------- OBJ models (scene ingestion)

@@ -310,12 +310,33 @@ pt_status pt_batch_autotune(pt_batch* b, uint32_t frames_per_trial, pt_tune_resu
   std::vector<uint32_t> trial_frames;
   for (uint32_t f : b->frames) trial_frames.push_back(std::min(f, frames_per_trial));
   const Options saved_opt = E.opt;
+  struct Restore {  // an error leaves the engine's options as they were
+    Options& o;
+    const Options& saved;
+    bool on;
+    ~Restore() { if (on) o = saved; }
+  } restore{E.opt, saved_opt, true};
   const uint64_t saved_max = E.max_paths;
   struct Cand { int mode, refill; uint64_t max_paths; };
   std::vector<Cand> cands;
   for (uint64_t mp : {1ull << 22, 1ull << 23, 1ull << 24})
     for (int r : {16, 20, 24}) cands.push_back({1, r, mp});
   cands.push_back({0, 20, 1ull << 23});
+  // Every trial runs on the schedule that a full render takes with the candidate's settings (a trial of fewer
+  // frames could fall under the pools' line and time a schedule that no render uses).
+  auto schedule = [&](bool& pools) -> pt_status {
+    E.opt.pool = saved_opt.pool;
+    PassLayout full;
+    std::vector<SceneDev> tab;
+    uint64_t samples = 0;
+    for (pt_ctx* s : b->scenes) s->c.next_frame = 0;
+    pt_status st = plan(b, full, tab, samples, nullptr);
+    if (st != PT_OK) return st;
+    pools = pass_by_pools(E.opt, full, tab);
+    E.opt.pool = pools ? 2 : 0;
+    return PT_OK;
+  };
+  bool pools = false;
   float best = 0.0f;
   Cand win = cands.front();
   uint32_t trials = 0;
@@ -323,8 +344,8 @@ pt_status pt_batch_autotune(pt_batch* b, uint32_t frames_per_trial, pt_tune_resu
     E.opt.extend_mode = cd.mode;
     E.opt.refill = cd.refill;
     E.max_paths = cd.max_paths;
-    for (size_t k = 0; k < b->scenes.size(); ++k) b->scenes[k]->c.next_frame = 0;
-    pt_status st = render(b, false, &trial_frames, false);  // warm (allocations, caches)
+    pt_status st = schedule(pools);
+    if (st == PT_OK) st = render(b, false, &trial_frames, false);  // warm (allocations, caches)
     if (st == PT_OK) st = render(b, false, &trial_frames, false);
     if (st != PT_OK) return st;
     PT_CHECK_CUDA(cudaStreamSynchronize(E.stream), "autotune");
@@ -337,13 +358,16 @@ pt_status pt_batch_autotune(pt_batch* b, uint32_t frames_per_trial, pt_tune_resu
       win = cd;
     }
   }
-  // second stage: the sort granularity (queue positions per binning thread) for the winner
+  // second stage: the sort granularity (queue positions per binning thread) for the winner, where its full
+  // render bins at all (path pools do not)
   int win_items = E.opt.bin_items;
   E.opt.extend_mode = win.mode;
   E.opt.refill = win.refill;
   E.max_paths = win.max_paths;
+  pt_status sst = schedule(pools);
+  if (sst != PT_OK) return sst;
   for (int items : {4, 16}) {
-    if (items == win_items) continue;
+    if (pools || items == win_items) continue;
     E.opt.bin_items = items;
     for (size_t k = 0; k < b->scenes.size(); ++k) b->scenes[k]->c.next_frame = 0;
     pt_status st = render(b, false, &trial_frames, false);
@@ -359,6 +383,7 @@ pt_status pt_batch_autotune(pt_batch* b, uint32_t frames_per_trial, pt_tune_resu
       win_items = items;
     }
   }
+  restore.on = false;
   E.opt = saved_opt;
   E.opt.extend_mode = win.mode;
   E.opt.refill = win.refill;

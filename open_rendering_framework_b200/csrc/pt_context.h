@@ -299,6 +299,10 @@ SceneFacts scene_facts(const Context& c);
 // dual: a pass without translucent materials is planned in chunks of at most max_paths / 2 paths that
 // launch_pass runs two at a time (PassLayout::dual).
 PassLayout plan_pass(const std::vector<SceneFacts>& facts, const std::vector<ItemReq>& reqs, uint64_t max_paths, bool dual = false);
+// Whether a chunk of n paths runs by path pools (multi: its paths belong to several scenes; w4: every scene
+// has the wide BVH), and whether most of a planned pass's paths do.
+bool chunk_by_pools(const Options& o, const PassLayout& L, uint64_t n, bool multi, bool w4);
+bool pass_by_pools(const Options& o, const PassLayout& L, const std::vector<SceneDev>& scenes);
 pt_status pass_resources(Context& E, const PassLayout& L, const std::vector<SceneDev>& scenes);
 pt_status launch_pass(Context& E, const PassLayout& L, const std::vector<SceneDev>& tab, bool multi, bool allow_events, bool adjoint = false);
 

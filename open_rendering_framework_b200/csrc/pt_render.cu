@@ -1465,6 +1465,36 @@ PassLayout plan_pass(const std::vector<SceneFacts>& facts, const std::vector<Ite
   return L;
 }
 
+// The scene whose paths alone chunk k of the pass holds, or -1.
+static int scene_of_chunk(const PassLayout& L, size_t k)
+{
+  const uint32_t ib = L.chunk_item_begin[k];
+  const uint32_t ie = k + 1 < L.chunk_paths.size() ? L.chunk_item_begin[k + 1] : (uint32_t)L.items.size();
+  for (uint32_t i = ib + 1; i < ie; ++i)
+    if (L.items[i].scene != L.items[ib].scene) return -1;
+  return (int)L.items[ib].scene;
+}
+static bool all_wide(const std::vector<SceneDev>& scenes)
+{
+  for (const SceneDev& s : scenes)
+    if (!s.nodes4) return false;
+  return true;
+}
+bool chunk_by_pools(const Options& o, const PassLayout& L, uint64_t n, bool multi, bool w4)
+{
+  return o.pool && w4 && o.extend_mode == 1 && (o.pool == 2 || n <= pool_max_paths(L.sss, L.ms || L.layered || L.rough, multi));
+}
+bool pass_by_pools(const Options& o, const PassLayout& L, const std::vector<SceneDev>& scenes)
+{
+  const bool w4 = all_wide(scenes);
+  uint64_t all = 0, pools = 0;
+  for (size_t k = 0; k < L.chunk_paths.size(); ++k) {
+    all += L.chunk_paths[k];
+    if (chunk_by_pools(o, L, L.chunk_paths[k], scenes.size() > 1 && scene_of_chunk(L, k) < 0, w4)) pools += L.chunk_paths[k];
+  }
+  return 2 * pools > all;
+}
+
 // Allocates what a pass needs in the engine context E and uploads its scene and item tables (on
 // E's stream).  Nothing here may run while E's stream is being captured.
 pt_status pass_resources(Context& E, const PassLayout& L, const std::vector<SceneDev>& scenes)
@@ -1480,8 +1510,7 @@ pt_status pass_resources(Context& E, const PassLayout& L, const std::vector<Scen
   if (st == PT_OK) st = E.d_scene_tab.reserve(scenes.size() * sizeof(SceneDev), "scene table");
   if (st == PT_OK) st = E.d_item_tab.reserve(std::max<size_t>(L.items.size(), 1) * sizeof(ItemDev), "item table");
   if (st != PT_OK) return st;
-  E.pass_w4 = true;
-  for (const SceneDev& s : scenes) E.pass_w4 = E.pass_w4 && s.nodes4 != nullptr;
+  E.pass_w4 = all_wide(scenes);
   // the overlapped schedule's streams and events (created here, outside any graph capture)
   for (cudaStream_t& sd : E.side)
     if (!sd) PT_CHECK_CUDA(cudaStreamCreateWithFlags(&sd, cudaStreamNonBlocking), "side stream");
@@ -1647,9 +1676,7 @@ pt_status launch_pass(Context& E, const PassLayout& L, const std::vector<SceneDe
     return PT_OK;
   };
   // a chunk of n paths runs its bounces by path pools
-  auto by_pools = [&](uint64_t n) {
-    return c.opt.pool && !prof && w4 && c.opt.extend_mode == 1 && (c.opt.pool == 2 || n <= pool_max_paths(L.sss, L.ms || L.layered || L.rough, multi));
-  };
+  auto by_pools = [&](uint64_t n) { return !prof && chunk_by_pools(c.opt, L, n, multi, w4); };
   const PoolPrograms programs = L.ms || L.layered || L.rough ? POOL_ALL : L.sss ? POOL_TRANSLUCENT : POOL_BASIC;
   // L.passes = max_depth + 2 bounces: every path has ended by then (each shader stops at max_depth).
   auto bounces = [&](uint64_t n, bool adj_pass) -> pt_status {
@@ -1760,9 +1787,7 @@ pt_status launch_pass(Context& E, const PassLayout& L, const std::vector<SceneDe
     const uint32_t ie = k + 1 < n_chunks ? L.chunk_item_begin[k + 1] : (uint32_t)L.items.size();
     w.items = items + ib;
     w.n_items = ie - ib;
-    bool one_scene = true;
-    for (uint32_t i = ib + 1; i < ie; ++i) one_scene = one_scene && L.items[i].scene == L.items[ib].scene;
-    multi = multi_pass && !one_scene;
+    multi = multi_pass && scene_of_chunk(L, k) < 0;
     w.multi = multi ? 1u : 0u;
     w.scene0 = multi ? 0u : L.items[ib].scene;
     S0 = tab[w.scene0];
