@@ -9,7 +9,7 @@ PT_D float3 sqrtf3(const float3& a) { return f3(sqrtf(a.x), sqrtf(a.y), sqrtf(a.
 PT_D float3 fmaxf3(const float3& a, const float3& b) { return f3(fmaxf(a.x, b.x), fmaxf(a.y, b.y), fmaxf(a.z, b.z)); }
 PT_D float3 operator+(float s, const float3& a) { return f3(s + a.x, s + a.y, s + a.z); }
 
-// The per-material terms of dipole_bssrdf (standard_dipole.h:10-13), hoisted out of the probe loop.
+// The per-material terms of dipole_bssrdf (standard_dipole.h:10-13), formed from the material by each caller.
 struct StdDipole {
   float3 three_D, transport, real_source, virtual_source, corrected_mean_free;
 };

@@ -18,16 +18,15 @@ namespace pt {
 // A path's arithmetic is that of the wavefront kernels (the same functions on the same records), and
 // the shadow ray of a vertex is added before the path's next vertex is shaded, so the images are the
 // wavefront's bit for bit.
-// What bounds it: a phase ends with its slowest ray (barrier stalls 6.3 per issue at 262 K paths), while
-// issue slots are 45 % busy; many small blocks in different phases evict each other's code instead (8
-// blocks of 128 threads: 8.5 fetch stalls per issue and 1.44 ms for a 512 x 512 frame, against 0.39 and
-// 0.93 ms here; 1.29 ms and 5.6 with twice the pool), and inlined draws did the same.
-// A 96 x 64 frame went from 776 to 272 us a pass, 512 x 512 from 900 to 589 (several contexts at once),
-// one frame of a translucent object from 1,026 to 476; pool_max_paths has the line to the wavefront.
+// What bounds it: a phase ends with its slowest ray (barrier stalls 5.7 per issue at 262 K paths), while
+// issue slots are 46 % busy.  Many small blocks in different phases evict each other's code instead (8 blocks
+// of 128 threads take half as long again), and so do inlined draws.  Against the wavefront's launches,
+// several contexts at once: a 96 x 64 frame 786 to 239 us, 512 x 512 879 to 567, one frame of a translucent object
+// 942 to 345; pool_max_paths has the line to the wavefront.
 //
 // Threads per block and places of a pool: two blocks of 512 threads per SM (64 registers) and, with all
 // vertex programs, one of 1,024, whose warps are all in the same phase: the large programs then share the
-// instruction cache (layered 301 x 203 x 6 with the multiple-scattering model: 4.5 ms against 5.5 ms).
+// instruction cache (layered scenes with the multiple-scattering model: 18 % less than two of 512).
 __host__ __device__ constexpr int pool_threads(int prog) { return prog == POOL_ALL ? 1024 : 512; }
 __host__ __device__ constexpr int pool_size(int prog) { return 4 * pool_threads(prog); }
 template <int kProg> struct PoolShared {
@@ -50,7 +49,7 @@ __device__ __forceinline__ void pool_trace(const SceneDev& S0, const WfDev& w, P
   TravGeom g = trav_geom(S0);
   const unsigned lane = threadIdx.x & 31;
   // few rays: each warp takes its share of them and no more, since the lanes of a warp take turns between
-  // nodes and leaves (a 96 x 64 frame alone: 280 to 257 us)
+  // nodes and leaves (a 96 x 64 frame alone: 8 % less)
   constexpr uint32_t kWarpsOfBlock = kPoolBlock / 32;
   const uint32_t lanes = min(32u, (n + kWarpsOfBlock - 1) / kWarpsOfBlock);
   const unsigned mine = lanes >= 32u ? 0xffffffffu : (1u << lanes) - 1u;
@@ -96,7 +95,7 @@ __device__ __forceinline__ void pool_trace(const SceneDev& S0, const WfDev& w, P
     if (__ballot_sync(0xffffffffu, has) == 0) break;
     for (;;) {
       // idle lanes have cur == kDone4, so the phase's two ballots also tell how many lanes have finished (a
-      // 96 x 64 frame alone 256 to 235 us; the wavefront's own loops lost 1 % to the same change)
+      // 96 x 64 frame alone: 8 % less; the wavefront's own loops lost 1 % to the same change)
       const bool lp = is_leaf4(cur), np = is_node4(cur);
       const unsigned lmask = __ballot_sync(0xffffffffu, lp), nmask = __ballot_sync(0xffffffffu, np), busy = lmask | nmask;
       if (busy == 0 || (!drained && __popc(mine & ~busy) >= refill)) break;

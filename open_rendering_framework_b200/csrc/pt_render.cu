@@ -642,9 +642,11 @@ __global__ void __launch_bounds__(kBlock) k_gather_collect(WfDev w, uint64_t n_p
 // dipole.  The sum times global_coeff / samples is added to the path's radiance, weighted by the
 // throughput at the vertex.  The MD5 stream of a path is one sequential chain, so a lane owns a path.
 //
-// What bounds it: the 64 MD5 steps are three ALU-pipe instructions each (logic, three-input add,
-// shift-and-add; 190 per draw counted by ncu), and the ALU pipe takes 64 lanes per clock and SM, so a
-// draw costs at least 3.0 clocks per SM.  The rest of a pair is kept off that pipe and out of the way:
+// What bounds it: issue to the two integer pipes.  The 64 MD5 steps are a logic operation, a three-operand sum
+// and a shift-and-add each: 190 ALU instructions per draw, 3.0 clocks of an SM at 64 lanes a clock, if all run
+// there.  With the sums on the FMA pipe (md5_u2_split) they are 134 ALU and 128 FMA instructions: at least
+// 2.1 clocks of either pipe, and 2.05 of the SM's four issue slots (128 lanes a clock).  The rest of a pair
+// is kept out of the way:
 //  * the roulette is decided from the draw's upper 31 bits against an upper bound of p taken with the
 //    approximate square root and exponential (gather_bound); only the pairs that this bound cannot
 //    reject (the accepted ones and about one in 10^4 more) go through the exact test, which alone
@@ -654,13 +656,12 @@ __global__ void __launch_bounds__(kBlock) k_gather_collect(WfDev w, uint64_t n_p
 //    then adds the values of its own pairs in probe order, so the sum is the sequential one bit for bit;
 //  * a lane whose path is done takes the next path of the list at once, and the warp steps through the
 //    pairs without any test of the lanes' ends until the first of them is due;
-//  * the next probe is loaded before the draw and bounded after it;
-//  * the draw's additions run on the FMA pipe (md5_u2_split).
-// One thread per path with the exact test in the probe loop and the dipole on the accepting lanes took
-// 19.6 ms for 456,028 gathers of 3,011 pairs (512 x 512 x 4 frames, 4,096 probes: 69.9 Gpair/s); this
-// takes 16.2 ms (84.8).  Gathers of few pairs and many acceptances (175,143 of 312 pairs, scale 10): 3.04
-// to 1.27 ms.  Six blocks per SM with the evaluation out of line: 5 blocks the same, 8 to 12 spill and are 2 to
-// 4 % slower.
+//  * the next probe is loaded before the draw and bounded after it.
+// 456,028 gathers of 3,011 pairs (512 x 512 x 4 frames, 4,096 probes): 16.4 ms, 84.0 Gpair/s, 302 thread
+// instructions a pair at 71 % of the issue slots, against 19.6 ms for one thread per path with the exact test in
+// the probe loop and the dipole on the accepting lanes; gathers of few pairs and many acceptances take less than
+// half of what they took so.  Six blocks per SM with the evaluation out of line: 5 blocks the same, 8 to 12
+// spill and are 2 to 4 % slower.
 //
 // A differentiable forward render also stores each gather's value with the path (adj_G).  kAdj: the
 // adjoint replays the same chain; a queued pair of a differentiated material adds the standard dipole's

@@ -144,8 +144,8 @@ __device__ __forceinline__ float3 shading_normal(const SceneDev& S, const int4& 
 }
 
 // Visibility for the vertex programs that trace a shadow ray of their own (one copy, out of line).  Over
-// the wide BVH where its box tests hold, as the shadow kernels: layered 301 x 203 x 6 with the
-// multiple-scattering model 3.72 to 2.55 ms a pass.
+// the wide BVH where its box tests hold, as the shadow kernels: a third less for a pass of layered objects with
+// the multiple-scattering model than over the BVH2.
 static __device__ __noinline__ bool occluded(const SceneDev& S, float3 o, float3 d, float tmin, float tmax)
 {
   const TravGeom g = trav_geom(S);
